@@ -97,24 +97,32 @@ fe::Pyr to_pyr(const fe_pyramid& p) {
 // memory together; each level before it is a banded phase (its gradients and the next level's
 // image, a band of rows per item).  False when no such split exists (the job then keeps the
 // generic stages).
+// Bands are short, about kBandPixels of the next level each, and a level above kRestPixels pixels is
+// banded even where the rest item could hold it: a small frame's time is the chain of its deeper levels,
+// which many CTAs then share.  One 1920x1200 frame takes 25.3 us with 256-pixel bands, 26.1 with 512,
+// 27.7 with 1024, and 27.0 when its level 4 stays in the rest item.
+constexpr int kRestPixels = 2048, kBandPixels = 256, kBandMinRows = 4;
 bool plan_deep_items(const fe::Pyr& pyr, fe::StageJob& job) {
   const int n = pyr.levels - 3, cap = fe::l012_deep_floats();
   if (n <= 0) return false;
   int r = -1;
   for (int k = 0; k < std::min(n, 3) && r < 0; ++k) {
     int64_t need = (int64_t)((pyr.lv[3 + k].w + 3) & ~3) * pyr.lv[3 + k].h;
-    for (int m = k + 1; m < n; ++m) need += (int64_t)pyr.lv[3 + m].w * pyr.lv[3 + m].h;
+    for (int m = k + 1; m < n; ++m) need += (int64_t)((pyr.lv[3 + m].w + 3) & ~3) * pyr.lv[3 + m].h;
     if (need <= cap) r = k;
   }
   if (r < 0) return false;
+  // a level that would keep the one rest item busy for long is banded too, so that several CTAs share it
+  while (r < 2 && r + 1 < n && pyr.lv[3 + r].w * pyr.lv[3 + r].h > kRestPixels) ++r;
   job.deep_rest = r;
   job.deep_bands[0] = job.deep_bands[1] = 0;
   job.deep_band_rows[0] = job.deep_band_rows[1] = 0;
   job.deep_items = 1;
   for (int p = 0; p < r; ++p) {
     const int ws = (pyr.lv[3 + p].w + 3) & ~3;
-    const int rows = (cap / ws - 6) / 2;  // level 3+p+1 rows per band: 2 rows + 6 halo rows staged each
+    int rows = (cap / ws - 6) / 2;  // level 3+p+1 rows per band: 2 rows + 6 halo rows staged each
     if (rows < 1) return false;
+    rows = std::min(rows, std::max(kBandMinRows, (kBandPixels + pyr.lv[4 + p].w - 1) / pyr.lv[4 + p].w));
     job.deep_band_rows[p] = rows;
     job.deep_bands[p] = (pyr.lv[4 + p].h + rows - 1) / rows;
     job.deep_items += job.deep_bands[p];
@@ -129,6 +137,7 @@ struct StageGroup {
   bool u8;
   int nl;
   bool tail;  // jobs whose last CTA computes the remaining levels (more shared memory)
+  bool lead;  // the first stage of FP32 builds (its own kernels)
   int kt;  // deepest-level tile of the generic stages (8 or 16)
   int tiles;
   fe::StageBatch batch;
@@ -160,17 +169,24 @@ int plan_pyramid(const void* src, int64_t src_pitch, bool u8, const fe_pyramid& 
     job.src_h = pyr.lv[s].h;
     for (int k = 0; k <= nl; ++k) job.out[k] = pyr.lv[s + k];
     const bool kind_u8 = stage == 0 && u8;
-    const int T = fe::stage_tile(kind_u8, nl, kt);
+    const bool lead = stage == 0 && !u8 && nl == 2;
+    job.keep_level0 = lead && src == (const void*)pyr.lv[0].img && src_pitch == (int64_t)pyr.lv[0].pitch * 4 &&
+                      scale == 1.f;
+    const int T = fe::stage_tile(kind_u8, nl, kt, lead);
     const fe::Level& deep = pyr.lv[s + nl];
     job.tiles_x = (deep.w + T - 1) / T;
     job.tiles_y = (deep.h + T - 1) / T;
     if (kind_u8 && nl == 2) fe::encode_frame_tmap(job);
+    if (lead) fe::encode_lead_tmap(job);
     const int rem = pyr.levels - 1 - (s + std::max(nl, 0));
     if (kind_u8 && nl == 2 && rem > 0 && counters && *ncounters + 4 <= counter_cap && plan_deep_items(pyr, job)) {
       // the levels 0-2 launch also computes every deeper level (work items after the tiles)
       job.done = counters + *ncounters;
       *ncounters += 4;
-    } else if (!(kind_u8 && nl == 2) && nl > 0 && rem > 0 && rem <= 2 && counters && *ncounters < counter_cap) {
+    } else if (lead && rem > 0 && ((pyr.lv[3].w + 3) & ~3) <= fe::lead_deep_max_width()) {
+      job.tail_levels = rem;
+      for (int k = 0; k < rem; ++k) job.tail[k] = pyr.lv[3 + k];
+    } else if (!lead && !(kind_u8 && nl == 2) && nl > 0 && rem > 0 && rem <= 2 && counters && *ncounters < counter_cap) {
       const fe::Level& deepest = pyr.lv[s + nl];
       const fe::Level& next = pyr.lv[s + nl + 1];
       if ((int64_t)deepest.w * deepest.h + (int64_t)next.w * next.h <= fe::kTailFloats) {
@@ -191,6 +207,7 @@ int plan_pyramid(const void* src, int64_t src_pitch, bool u8, const fe_pyramid& 
       g->u8 = kind_u8;
       g->nl = nl;
       g->tail = has_tail;
+      g->lead = lead;
       g->kt = kt;
       g->tiles = 0;
     }
@@ -206,7 +223,9 @@ int plan_pyramid(const void* src, int64_t src_pitch, bool u8, const fe_pyramid& 
 // The launches of stages [first, last) of a plan.
 int run_stages(const StagePlan& plan, size_t first, size_t last, cudaStream_t st) {
   for (size_t k = first; k < std::min(last, plan.size()); ++k)
-    for (const auto& g : plan[k]) FE_CUDA(fe::launch_pyramid_stage(g.batch, g.tiles, g.u8, g.nl, g.kt, g.tail, st));
+    for (const auto& g : plan[k])
+      FE_CUDA(g.lead ? fe::launch_pyramid_lead(g.batch, g.tiles, g.tail, st)
+                     : fe::launch_pyramid_stage(g.batch, g.tiles, g.u8, g.nl, g.kt, g.tail, st));
   return FE_OK;
 }
 
@@ -242,11 +261,7 @@ int finish_l012_plan(StagePlan& plan, int* queues, int* nqueues, int queue_cap) 
   return FE_OK;
 }
 
-int run_plan(const StagePlan& plan, cudaStream_t st) {
-  for (const auto& stage : plan)
-    for (const auto& g : stage) FE_CUDA(fe::launch_pyramid_stage(g.batch, g.tiles, g.u8, g.nl, g.kt, g.tail, st));
-  return FE_OK;
-}
+int run_plan(const StagePlan& plan, cudaStream_t st) { return run_stages(plan, 0, plan.size(), st); }
 
 }  // namespace
 
@@ -1923,7 +1938,8 @@ int fe_adjoint_kernel_count(const fe_adjoint* a, int backward) {
   if (!a) return -1;
   if (backward == 2) {  // pyramid builds
     int n = 0;
-    for (const auto& stage : a->build) n += (int)stage.size();
+    for (const auto& stage : a->build)
+      for (const auto& g : stage) n += g.lead && g.tail ? 2 : 1;
     return n;
   }
   if (!backward) return a->total > 0 ? 1 : 0;

@@ -17,6 +17,7 @@ struct alignas(64) StageJob {
   int src_w, src_h;
   int write_level0;         // also write level s (image cast + gradients): the uint8 stage
   int use_tma;              // frame meets TMA alignment (16-byte base and pitch)
+  int keep_level0;          // the source is level 0's own plane: its image is not rewritten
   float scale;              // factor on the staged source (FP32 first stage; 1 otherwise)
   int box3;                 // levels 0-2 kernel: apply the box prefilter to the uint8 frame
   int tiles_x, tiles_y;
@@ -54,17 +55,23 @@ static_assert(sizeof(StageBatch) <= 32000, "stage job table exceeds the kernel p
 // kt: the generic stages' deepest-level tile (8 or 16), plus kL012Three to run the levels 0-2 kernel
 // with registers for three CTAs per SM instead of two
 constexpr int kL012Three = 64;
-int stage_tile(bool u8, int nl, int kt);  // deepest-level core tile edge of a stage kind
+int stage_tile(bool u8, int nl, int kt, bool lead);  // deepest-level core tile edge of a stage kind
+int lead_deep_max_width();  // widest level 3 whose rows the FP32 deeper-level kernel can stage
 constexpr int kTailFloats = 12 * 1024;  // shared-memory floats for a tail: the source level + one level
 int l012_deep_floats();  // shared-memory floats a deeper-level item of the levels 0-2 kernel stages
 // Encodes the uint8 frame's tensor map into job.tmap; returns false when the frame does not meet
 // TMA alignment (the stage then stages its tile with ordinary loads).
 bool encode_frame_tmap(StageJob& job);
+// The same for an FP32 frame's first stage.
+bool encode_lead_tmap(StageJob& job);
 // Encodes a 2-D FP32 plane's tensor map (w x h floats, rows pitch_floats apart) with a box of
 // box_w x box_h floats; false when the driver entry point is missing or the plane does not meet TMA
 // alignment (16-byte base and pitch).
 bool encode_plane_tmap_f32(CUtensorMap* map, const float* base, int w, int h, int pitch_floats, int box_w, int box_h);
 cudaError_t pyramid_init();  // kernel attributes; call once per device before capture
+// The first stage of FP32 builds of three or more levels: levels 0-2 and, with `tail`, level 3's image
+// and then every deeper level in a second launch.
+cudaError_t launch_pyramid_lead(const StageBatch& b, int tiles, bool tail, cudaStream_t s);
 cudaError_t launch_pyramid_stage(const StageBatch& b, int tiles, bool u8, int nl, int kt, bool tail, cudaStream_t s);
 // Level 0 of a pyramid from a uint8 mono (channels 1) or RGB8 (channels 3) frame: the reference's cast
 // (gray = 0.299 r + 0.587 g + 0.114 b for RGB) and, with box3, its box prefilter; FP32 into dst.
