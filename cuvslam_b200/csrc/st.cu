@@ -14,11 +14,18 @@
 // (tap f = lane + 32 e, e < 3); each lane samples its taps straight from global memory (4 texels per
 // plane, clamped, one bilinear set-up shared by the image and both gradients; the texture unit's
 // weight rule emulated as in the LK tracker).  A patch sum is a lane-major partial sum then an xor
-// butterfly; the 19 moments of a full step are summed by recursive halving (value k ends in lane k,
-// each addition pairing the same partial sums as the butterfly) and gathered straight into the
-// columns of the 6x6 system.  The QR solve is spread over the warp: lane c holds column c, lane D the
-// right side, so each reflector and norm update runs once per column in parallel.  Operations are
-// unfused (__fmul_rn / __fadd_rn) so the oracle restates them exactly.
+// butterfly; the 24 sums of a full step share one by recursive halving (value k ends in lane k, each
+// addition pairing the same partial sums as the butterfly) and are gathered straight into the columns
+// of the 6x6 system.  The QR solve is spread over the warp: lane c holds column c, lane D the right side,
+// so each reflector and norm update runs once per column in parallel.  Operations are unfused
+// (__fmul_rn / __fadd_rn) so the oracle restates them exactly.
+//
+// Bound by issue with many tracks and by a track's chain of steps with few (a step of one warp alone:
+// 10 800 cycles before the sums shared a butterfly, the QR's steps were unrolled and its pivot found by a
+// warp maximum, 6 400 of them in the QR).  1920x1200, 20 full steps a level: 150 tracks 574 -> 438 us,
+// 2400 tracks 852 -> 586, 8191 tracks 1716 -> 1519.  Several tracks per warp or block with their QR solves
+// side by side were slower (1.8-5.1 ms at 8191): their code and their barriers cost more than the idle
+// lanes of one solve.
 #include <cuda_runtime.h>
 
 #include "fe_common.cuh"
@@ -32,10 +39,6 @@ namespace {
 using lk::kFull;
 using lk::Tap;
 constexpr int kWarps = 8;
-#ifndef FE_ST_MIN_BLOCKS
-#define FE_ST_MIN_BLOCKS 3  // tracking blocks per SM the register budget is sized for (80 registers)
-#endif
-constexpr int kMinBlocks = FE_ST_MIN_BLOCKS;
 constexpr float kEps = 1.1920928955078125e-07f;
 
 // Bilinear set-up of one sample at texture coordinate (x, y) of a level: the four clamped texel
@@ -151,24 +154,14 @@ __device__ bool qr_solve_warp(float (&col)[D], int lane, float (&z)[D]) {
   float th = __fmul_rn(max_norm, kEps);
   th = __fdiv_rn(__fmul_rn(th, th), (float)D);
   int nzp = D;
-#pragma unroll 1
+#pragma unroll
   for (int q = 0; q < D - 1; ++q) {
     // pivot: the largest remaining column norm, the first column on ties
-    float key = (lane >= q && is_col && cn > -1.f) ? cn : -1.f;
-    int idx = lane;
-#pragma unroll
-    for (int m = 1; m < 8; m <<= 1) {
-      const float ok = __shfl_xor_sync(kFull, key, m);
-      const int oi = __shfl_xor_sync(kFull, idx, m);
-      if (ok > key || (ok == key && oi < idx)) {
-        key = ok;
-        idx = oi;
-      }
-    }
-    key = __shfl_sync(kFull, key, 0);
-    idx = __shfl_sync(kFull, idx, 0);
-    const int mc = key > -1.f ? idx : -1;
-    float mn = key > -1.f ? key : -1.f;
+    // (a norm is never negative, so its bits order as it does; 0 stands for a NaN or no column)
+    const unsigned key = lane >= q && is_col && cn > -1.f ? __float_as_uint(cn) + 1u : 0u;
+    const unsigned best = __reduce_max_sync(kFull, key);
+    const int mc = best ? __ffs(__ballot_sync(kFull, key == best)) - 1 : -1;
+    float mn = best ? __uint_as_float(best - 1u) : -1.f;
     if (nzp == D && __fmul_rn(mn, mn) < __fmul_rn(th, (float)(D - q))) nzp = q;
     if (mc >= 0 && mc != q) {
       const int src = lane == q ? mc : (lane == mc ? q : lane);
@@ -245,11 +238,11 @@ __device__ bool qr_solve_warp(float (&col)[D], int lane, float (&z)[D]) {
   return true;
 }
 
-// Slots of the 19 full-step moments after reduce_scatter: moment (m, c) of position weight m
+// Slots of the full step's moments after reduce_scatter: moment (m, c) of position weight m
 // (1 x, 2 y, 3 x^2, 4 xy, 5 y^2) and gradient product c (0 gx gx, 1 gx gy, 2 gy gy) in slot
 // 3 (m - 1) + c; the residual moments (x gx, x gy, y gx, y gy) in slots 15-18.  Row r of column c of
 // the symmetric 6x6 system in the reference's layout (st_tracker.cu:632-636), and b in column 6; 31
-// marks the moments with weight 1 (held by every lane).
+// marks the moments with weight 1 (slots 19-23, which every lane holds).
 constexpr int kColSlot[7][6] = {{6, 7, 9, 10, 0, 1},    {7, 8, 10, 11, 1, 2},   {9, 10, 12, 13, 3, 4},
                                 {10, 11, 13, 14, 4, 5}, {0, 1, 3, 4, 31, 31},   {1, 2, 4, 5, 31, 31},
                                 {15, 16, 17, 18, 31, 31}};
@@ -376,27 +369,21 @@ __device__ bool refine(const Level& L, const float* prev, float prev_sum, int n_
         p[e] = gx[e] = gy[e] = 0.f;
       }
     }
-    const float cs = TAP_SUM(T, p[e]), gxs = TAP_SUM(T, gx[e]), gys = TAP_SUM(T, gy[e]);
-    const float delta = __fdiv_rn(__fsub_rn(cs, prev_sum), 81.f);
-    const float gxm = __fdiv_rn(gxs, 81.f), gym = __fdiv_rn(gys, 81.f);
+    float cs = LANE_SUM(T, p[e]), gxs = LANE_SUM(T, gx[e]), gys = LANE_SUM(T, gy[e]);
+    warp_sum3(cs, gxs, gys, lane);
+    const float mean = __fdiv_rn(lane == 0 ? __fsub_rn(cs, prev_sum) : lane == 1 ? gxs : gys, 81.f);
+    const float delta = __shfl_sync(kFull, mean, 0), gxm = __shfl_sync(kFull, mean, 1),
+                gym = __shfl_sync(kFull, mean, 2);
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
       gx[e] = __fsub_rn(gx[e], gxm);
       gy[e] = __fsub_rn(gy[e], gym);
       r[e] = __fsub_rn(__fsub_rn(p[e], prev[e]), delta);
     }
-    const float sxx = TAP_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gx[e]), gx[e]));
-    const float sxy = TAP_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gx[e]), gy[e]));
-    const float syy = TAP_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gy[e]), gy[e]));
-    const float rx = TAP_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], r[e]), gx[e]));
-    const float ry = TAP_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], r[e]), gy[e]));
-    const float det = __fsub_rn(__fmul_rn(sxx, syy), __fmul_rn(sxy, sxy));
-    const float vx = __fdiv_rn(__fsub_rn(__fmul_rn(syy, rx), __fmul_rn(sxy, ry)), det);
-    const float vy = __fdiv_rn(__fsub_rn(__fmul_rn(sxx, ry), __fmul_rn(sxy, rx)), det);
-    s.converged = __fsqrt_rn(__fadd_rn(__fmul_rn(vx, vx), __fmul_rn(vy, vy))) < 0.04f;
-    if (s.converged) break;
+    float part[24];
+#pragma unroll
+    for (int k = 0; k < 24; ++k) part[k] = 0.f;
     if (full) {
-      float part[19];
 #pragma unroll
       for (int k = 1; k < 6; ++k) {
 #pragma unroll
@@ -418,7 +405,23 @@ __device__ bool refine(const Level& L, const float* prev, float prev_sum, int n_
         part[15 + k] = LANE_SUM(
             T, __fmul_rn(__fmul_rn(r[e], __fmul_rn(k < 2 ? (float)(T.ix[e] - 4) : (float)(T.iy[e] - 4), T.wt[e])),
                          (k % 2 == 0) ? gx[e] : gy[e]));
-      const float slot = reduce_scatter(part, lane);
+    }
+    part[19] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gx[e]), gx[e]));
+    part[20] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gx[e]), gy[e]));
+    part[21] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gy[e]), gy[e]));
+    part[22] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], r[e]), gx[e]));
+    part[23] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], r[e]), gy[e]));
+    const float slot = reduce_scatter(part, lane);
+    const float sxx = __shfl_sync(kFull, slot, 19), sxy = __shfl_sync(kFull, slot, 20),
+                syy = __shfl_sync(kFull, slot, 21), rx = __shfl_sync(kFull, slot, 22), ry = __shfl_sync(kFull, slot, 23);
+    const float det = __fsub_rn(__fmul_rn(sxx, syy), __fmul_rn(sxy, sxy));
+    const float nx = __fsub_rn(__fmul_rn(syy, rx), __fmul_rn(sxy, ry));
+    const float ny = __fsub_rn(__fmul_rn(sxx, ry), __fmul_rn(sxy, rx));
+    const float vv = __fdiv_rn(lane & 1 ? ny : nx, det);
+    const float vx = __shfl_sync(kFull, vv, 0), vy = __shfl_sync(kFull, vv, 1);
+    s.converged = __fsqrt_rn(__fadd_rn(__fmul_rn(vx, vx), __fmul_rn(vy, vy))) < 0.04f;
+    if (s.converged) break;
+    if (full) {
       float col[6], z[6];
       const int c = lane < 7 ? lane : 0;
 #pragma unroll
@@ -584,8 +587,9 @@ __device__ void track_one(const StLaunch& P, fe_track_data& td, const Taps& T, i
 }
 
 // Persistent warps: each takes the next track from P.counter (zeroed before the launch).
-template <int SAMPLING, bool CACHED>
-__global__ void __launch_bounds__(kWarps * 32, kMinBlocks) st_track_kernel(const __grid_constant__ StLaunch P) {
+// MINB: blocks per SM the registers are budgeted for.
+template <int SAMPLING, bool CACHED, int MINB>
+__global__ void __launch_bounds__(kWarps * 32, MINB) st_track_kernel(const __grid_constant__ StLaunch P) {
   const int lane = threadIdx.x & 31;
   const Taps T = make_taps(lane);
   for (;;) {
@@ -638,20 +642,33 @@ __global__ void __launch_bounds__(kWarps * 32) st_build_kernel(const __grid_cons
   }
 }
 
-template <int SAMPLING, bool CACHED>
-cudaError_t launch_track(const StLaunch& p, cudaStream_t s) {
-  // blocks resident on the device (persistent grid), found once per process
+// Blocks resident on the device (persistent grid), found once per process.
+template <int SAMPLING, bool CACHED, int MINB>
+int resident_blocks() {
   static const int resident = [] {
     int per_sm = 0, dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, st_track_kernel<SAMPLING, CACHED>, kWarps * 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, st_track_kernel<SAMPLING, CACHED, MINB>, kWarps * 32, 0);
     return (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
   }();
+  return resident;
+}
+
+template <int SAMPLING, bool CACHED>
+cudaError_t launch_track(const StLaunch& p, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(p.counter, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
-  const int blocks = min((p.n + kWarps - 1) / kWarps, resident);
-  st_track_kernel<SAMPLING, CACHED><<<blocks, kWarps * 32, 0, s>>>(p);
+  // While a warp at two blocks per SM (128 registers, no spills) has hardly more than a track of its own
+  // the chain of steps sets the time: 438 us there, 486 at three blocks (80 registers) with 150 tracks,
+  // 586 and 714 with 2400, 1029 both with 4800.  Past that the third block's warps pay: 1519 us against
+  // 1568 with 8191.
+  const int blocks = (p.n + kWarps - 1) / kWarps, two = resident_blocks<SAMPLING, CACHED, 2>();
+  if (2 * blocks <= 3 * two)
+    st_track_kernel<SAMPLING, CACHED, 2><<<min(blocks, two), kWarps * 32, 0, s>>>(p);
+  else
+    st_track_kernel<SAMPLING, CACHED, 3>
+        <<<min(blocks, resident_blocks<SAMPLING, CACHED, 3>()), kWarps * 32, 0, s>>>(p);
   return cudaGetLastError();
 }
 
