@@ -276,7 +276,6 @@ struct SelectScratch {
   float* cell_m = nullptr;
   float2* cell_xy = nullptr;
   float* sub_sum = nullptr;
-  int* bin_want = nullptr;
   int* stats = nullptr;
   uint64_t* q_keys = nullptr;
   float* alive_xy = nullptr;
@@ -380,7 +379,7 @@ int lk_textures(fe_context* ctx, const fe_pyramid& prev, const fe_pyramid& cur, 
 namespace {
 
 struct ScratchLayout {
-  size_t burn, cell_m, cell_xy, sub_sum, bin_want, stats, q_keys, alive, total, burn_bytes;
+  size_t burn, cell_m, cell_xy, sub_sum, stats, q_keys, alive, total, burn_bytes;
 };
 
 ScratchLayout scratch_layout(int w, int h, int n_alive_cap, int q_cap) {
@@ -394,13 +393,12 @@ ScratchLayout scratch_layout(int w, int h, int n_alive_cap, int q_cap) {
   const size_t words = (size_t)((w + 31) / 32) * h;
   const size_t cells = (size_t)(w / 8) * (h / 8);
   const size_t subs = (size_t)((w + 15) / 16) * ((h + 15) / 16);
-  L.stats = take(16 * sizeof(int));  // first so one memset clears stats + burn
+  L.stats = take(fe::kSelectStats * sizeof(int));  // first so one memset clears stats + burn
   L.burn = take(words * 4);
   L.burn_bytes = L.burn + words * 4;
   L.cell_m = take(std::max<size_t>(cells, 1) * 4);
   L.cell_xy = take(std::max<size_t>(cells, 1) * 8);
   L.sub_sum = take(subs * 4);
-  L.bin_want = take(128 * 4);
   L.q_keys = take((size_t)std::max(q_cap, 1) * 8);
   L.alive = take((size_t)std::max(n_alive_cap, 1) * 8);
   L.total = o;
@@ -448,7 +446,6 @@ int ensure_select_scratch(fe_context* ctx, int w, int h, int n_alive_cap, int q_
   s.cell_m = (float*)(base + L.cell_m);
   s.cell_xy = (float2*)(base + L.cell_xy);
   s.sub_sum = (float*)(base + L.sub_sum);
-  s.bin_want = (int*)(base + L.bin_want);
   s.q_keys = (uint64_t*)(base + L.q_keys);
   s.alive_xy = (float*)(base + L.alive);
   s.zero_bytes = L.burn_bytes;
@@ -471,7 +468,6 @@ void fill_select_cam(fe::SelectCam& c, const SelectScratch& s, const fe_pyramid&
   c.cell_m = s.cell_m;
   c.cell_xy = s.cell_xy;
   c.sub_sum = s.sub_sum;
-  c.bin_want = s.bin_want;
   c.stats = s.stats;
   c.q_keys = s.q_keys;
   c.q_cap = q_cap;
@@ -1353,7 +1349,7 @@ int fe_batch_create(fe_context* ctx, const fe_camera_frame* cams, int ncams, int
   // selection scratch: every camera's [stats | burn | touched] first (one memset per step), then
   // each camera's cells, sub-tile sums, quotas, kept keys and response/NMS maps
   struct BatchSel {
-    size_t stats, burn, touched, zero, cell_m, cell_xy, sub_sum, bin_want, q_keys, resp, rest;
+    size_t stats, burn, touched, zero, cell_m, cell_xy, sub_sum, q_keys, resp, rest;
     int touched_words;
   };
   std::vector<BatchSel> lay(ncams);
@@ -1382,7 +1378,7 @@ int fe_batch_create(fe_context* ctx, const fe_camera_frame* cams, int ncams, int
       o = (size_t)align_up((int64_t)(o + bytes), kAlign);
       return at;
     };
-    L.stats = take(16 * sizeof(int));
+    L.stats = take(fe::kSelectStats * sizeof(int));
     L.burn = take((size_t)((w + 31) / 32) * h * 4);
     L.touched = take((size_t)L.touched_words * 4);
     L.zero = o;
@@ -1390,7 +1386,6 @@ int fe_batch_create(fe_context* ctx, const fe_camera_frame* cams, int ncams, int
     L.cell_m = take(cells * 4);
     L.cell_xy = take(cells * 8);
     L.sub_sum = take((size_t)((w + 15) / 16) * ((h + 15) / 16) * 4);
-    L.bin_want = take(128 * 4);
     L.q_keys = take((size_t)std::max(qc, 1) * 8);
     L.resp = take((size_t)w * h * 4);  // the response map that cells_kernel reads
     L.rest = o;
@@ -1419,7 +1414,6 @@ int fe_batch_create(fe_context* ctx, const fe_camera_frame* cams, int ncams, int
       s.cell_m = (float*)(rp + L.cell_m);
       s.cell_xy = (float2*)(rp + L.cell_xy);
       s.sub_sum = (float*)(rp + L.sub_sum);
-      s.bin_want = (int*)(rp + L.bin_want);
       s.q_keys = (uint64_t*)(rp + L.q_keys);
       s.resp = (float*)(rp + L.resp);
       s.nms = nullptr;

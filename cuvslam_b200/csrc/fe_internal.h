@@ -79,6 +79,8 @@ cudaError_t launch_input_stage(const uint8_t* src, int64_t src_pitch, int channe
                                float* dst, int64_t dst_pitch_floats, cudaStream_t s);
 
 // ---------------------------------------------------------------- selection
+constexpr int kSelectBins = 16, kSelectStats = kSelectBins + 64;
+
 struct SelectCam {
   // level-0 gradients
   const float* gx;
@@ -89,9 +91,8 @@ struct SelectCam {
   const float* alive_xy;        // alive features as n_alive (x, y) pairs, or
   const fe_track_data* alive_tracks;  // n_alive tracks; alive = track_status != 0
   int n_alive;
-  float* alive_out_xy;          // optional: compacted alive positions (capacity n_alive)
-  int* stats;                   // [0] alive count, [1] quota total, [2] kept, [3] error flags,
-                                // [4] new features wanted
+  int* stats;                   // kSelectStats counters, zeroed before the launch: [0] alive count,
+                                // [2] kept, [3] error flags, [kSelectBins ..] alive features per bin
   int num_desired;              // new features wanted, or
   int target_total;             // when > 0: wanted = max(0, target_total - alive count)
   int border[4];
@@ -106,7 +107,6 @@ struct SelectCam {
   float* cell_m;                // (w/8)*(h/8) cell strength (0 = none)
   float2* cell_xy;              // refined position
   float* sub_sum;               // ceil(w/16)*ceil(h/16) sub-tile sums
-  int* bin_want;                // 64 quotas + 64 counts
   uint64_t* q_keys;             // qualifying keys, capacity q_cap
   float2* q_xy;
   int q_cap;

@@ -30,14 +30,14 @@ constexpr int kMaxKept = 16384;  // kept candidates: min(cells, n_alive + num_de
 constexpr size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 struct Layout {
-  size_t stats, burn, zero_end, cell_m, cell_xy, sub_sum, bin_want, q_keys, total;
+  size_t stats, burn, zero_end, cell_m, cell_xy, sub_sum, q_keys, total;
 };
 
 constexpr Layout layout(int w, int h, int q_cap) {
   Layout L{};
   size_t o = 0;
   L.stats = o;
-  o = align256(o + 16 * sizeof(int));
+  o = align256(o + fe::kSelectStats * sizeof(int));
   L.burn = o;
   o = align256(o + (size_t)((w + 31) / 32) * h * 4);
   L.zero_end = o;  // [0, zero_end) must be zero before every call
@@ -47,8 +47,6 @@ constexpr Layout layout(int w, int h, int q_cap) {
   o = align256(o + (size_t)(w / 8) * (h / 8) * 8 + 8);
   L.sub_sum = o;
   o = align256(o + (size_t)((w + 15) / 16) * ((h + 15) / 16) * 4);
-  L.bin_want = o;
-  o = align256(o + 128 * 4);
   L.q_keys = o;
   o = align256(o + (size_t)q_cap * 8);
   L.total = o;
@@ -165,7 +163,6 @@ extern "C" FE_API int fe_select_noalloc(const fe_pyramid* pyr, int border_top, i
   c.cell_m = (float*)(s + L.cell_m);
   c.cell_xy = (float2*)(s + L.cell_xy);
   c.sub_sum = (float*)(s + L.sub_sum);
-  c.bin_want = (int*)(s + L.bin_want);
   c.q_keys = (uint64_t*)(s + L.q_keys);
   c.q_cap = q_cap;
   c.tiles_x = (w + fe::select_tile_w() - 1) / fe::select_tile_w();
