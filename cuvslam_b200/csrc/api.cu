@@ -751,6 +751,7 @@ int fe_track_mono(fe_context* ctx, const fe_pyramid* prev, const fe_pyramid* cur
   p.single.tracks = tracks;
   p.single.n = n;
   p.single.retrack_ncc = retrack_ncc > 0.f ? retrack_ncc : 0.f;
+  p.retrack = retrack_ncc > 0.f;
   if (sampling == FE_SAMPLE_HARDWARE) {
     const int rc = lk_textures(ctx, *prev, *cur, false, p.single_tex);
     if (rc) return rc;
@@ -1295,6 +1296,7 @@ int fe_batch_create(fe_context* ctx, const fe_camera_frame* cams, int ncams, int
     b->lk.ncams = (int)lk.size();
     b->lk.total = total;
     b->lk.horizontal = 0;
+    for (const auto& c : lk) b->lk.retrack |= c.retrack_ncc > 0.f;
     b->lk.sampling = sampling;
     if (sampling == FE_SAMPLE_HARDWARE) {
       e = dev_alloc((void**)&b->d_tex, sizeof(fe::LkTex) * lk_tex.size());

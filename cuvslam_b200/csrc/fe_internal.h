@@ -171,6 +171,7 @@ struct LkLaunch {
   int ncams;
   int total;
   int horizontal;
+  int retrack;                  // some camera's retrack_ncc > 0
   int sampling;
   int mode;                     // kLk*
   int iters;                    // implicit: refinement steps at level 0; unrolled: steps per level

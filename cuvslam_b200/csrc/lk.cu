@@ -65,18 +65,20 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) lk_kernel(const __grid_const
         reinterpret_cast<uint32_t*>(&td)[lane] = reinterpret_cast<const uint32_t*>(&cam.tracks_in[g - cam.begin])[lane];
       __syncwarp();
     }
-    track_one<SAMPLING, HORIZ, MODE>(cam, td, smem[wid], lane, p.iters, p.tol2,
-                                     MODE == kModeUnrolled && p.recs ? p.recs + g : nullptr, p.counts);
-    if (MODE == kModeRef && cam.retrack_ncc > 0.f) {
+    const bool differs = track_one<SAMPLING, HORIZ, MODE>(
+        cam, td, smem[wid], lane, p.iters, p.tol2, MODE == kModeUnrolled && p.recs ? p.recs + g : nullptr, p.counts,
+        cam.retrack_ncc);
+    if (MODE == kModeRetrack && cam.retrack_ncc > 0.f && differs) {
       // MonoSOFGPU's retrack pass, merged as collect reads it: a track the first pass lost (its
-      // record still holds the inputs) runs again with the retrack NCC threshold
+      // record still holds the inputs) runs again with the retrack NCC threshold, when that threshold
+      // changes a gate's decision
       __syncwarp();
       if (td.track_status == 0 && td.search_radius_px >= 0.f) {
         const float keep = td.ncc_threshold;
         __syncwarp();
         if (lane == 0) td.ncc_threshold = cam.retrack_ncc;
         __syncwarp();
-        track_one<SAMPLING, HORIZ, MODE>(cam, td, smem[wid], lane, p.iters, p.tol2, nullptr, p.counts);
+        track_one<SAMPLING, HORIZ, kModeRef>(cam, td, smem[wid], lane, p.iters, p.tol2, nullptr, p.counts);
         __syncwarp();
         if (lane == 0) td.ncc_threshold = keep;
       }
@@ -105,7 +107,7 @@ cudaError_t launch_shape(const LkLaunch& p, cudaStream_t s) {
 // the first.
 template <int SAMPLING, bool HORIZ, int MODE>
 cudaError_t launch(const LkLaunch& p, cudaStream_t s) {
-  if (MODE == kModeRef) {
+  if (MODE == kModeRef || MODE == kModeRetrack) {
     switch (p.shape) {
       case 1: return launch_shape<SAMPLING, HORIZ, MODE, 8, 3>(p, s);
       case 2: return launch_shape<SAMPLING, HORIZ, MODE, 4, 8>(p, s);
@@ -127,6 +129,11 @@ cudaError_t launch_lk(const LkLaunch& p, cudaStream_t s) {
   }
   if (p.mode == kLkImplicit) return launch<FE_SAMPLE_EXACT, false, kModeImplicit>(p, s);
   if (p.mode == kLkUnrolled) return launch<FE_SAMPLE_EXACT, false, kModeUnrolled>(p, s);
+  if (p.retrack) {  // (horizontal launches have no retrack pass)
+    if (p.sampling == FE_SAMPLE_EXACT) return launch<FE_SAMPLE_EXACT, false, kModeRetrack>(p, s);
+    if (p.sampling == FE_SAMPLE_TEXTURE_WIDE) return launch<FE_SAMPLE_TEXTURE_WIDE, false, kModeRetrack>(p, s);
+    return launch<FE_SAMPLE_TEXTURE, false, kModeRetrack>(p, s);
+  }
   if (p.sampling == FE_SAMPLE_EXACT)
     return p.horizontal ? launch<FE_SAMPLE_EXACT, true, kModeRef>(p, s) : launch<FE_SAMPLE_EXACT, false, kModeRef>(p, s);
   if (p.sampling == FE_SAMPLE_TEXTURE_WIDE)

@@ -18,15 +18,18 @@ namespace lk {
 // settle within `iters` steps, takes a step or drifts beyond 2 px, or ends where J is ill
 // conditioned); and kModeUnrolled: exactly `iters` steps on
 // every level (no early stop), the level accepted when the last |v| < 0.12 and the gates pass.
-constexpr int kModeRef = 0, kModeImplicit = 1, kModeUnrolled = 2;
+// kModeRetrack is kModeRef for launches with a retrack pass: it also notes whether that pass would differ.
+constexpr int kModeRef = 0, kModeImplicit = 1, kModeUnrolled = 2, kModeRetrack = 3;
 
 // `rec` (unrolled mode only, may be null) receives the per-level record the adjoint replays.
 // `cnt` (may be null) counts the work done: [0] levels set up (previous patch and gradients sampled,
 // Hessian formed), [1] Gauss-Newton steps (current patch sampled, update solved), [2] NCC
-// evaluations.
+// evaluations.  Returns whether a level's NCC gate would have decided otherwise with the threshold
+// ncc_other (kModeRetrack): while none does, a run with that threshold ends the same way.
 template <int SAMPLING, bool HORIZ, int MODE>
-__device__ void track_one(const LkCam& cam, fe_track_data& td, WarpSmem& sm, int lane, int iters, float tol2,
-                          LkRecord* rec = nullptr, unsigned long long* cnt = nullptr) {
+__device__ bool track_one(const LkCam& cam, fe_track_data& td, WarpSmem& sm, int lane, int iters, float tol2,
+                          LkRecord* rec = nullptr, unsigned long long* cnt = nullptr, float ncc_other = 0.f) {
+  bool differs = false;
   if (MODE == kModeUnrolled && rec) {
     if (lane < kMaxLevels) rec->flags[lane] = 0;
     __syncwarp();
@@ -36,7 +39,7 @@ __device__ void track_one(const LkCam& cam, fe_track_data& td, WarpSmem& sm, int
   if (radius < 0.f) {
     __syncwarp();
     if (lane == 0) td.track_status = 0;
-    return;
+    return differs;
   }
   const float tx = td.track[0], ty = td.track[1];
   const float cx0 = __fadd_rn(tx, td.offset[0]), cy0 = __fadd_rn(ty, td.offset[1]);
@@ -49,7 +52,7 @@ __device__ void track_one(const LkCam& cam, fe_track_data& td, WarpSmem& sm, int
   const float CW0 = (float)cam.cur.lv[0].w, CH0 = (float)cam.cur.lv[0].h;
   if (!(tx >= 0.f && tx < W0 && ty >= 0.f && ty < H0) || !(cx0 >= 0.f && cx0 < CW0 && cy0 >= 0.f && cy0 < CH0)) {
     if (lane == 0) td.track_status = 0;
-    return;
+    return differs;
   }
   const float scale = 1.f / (float)(1 << top);
   float sx = __fmaf_rn(__fsub_rn(tx, 0.5f), scale, 0.5f), sy = __fmaf_rn(__fsub_rn(ty, 0.5f), scale, 0.5f);
@@ -158,14 +161,14 @@ __device__ void track_one(const LkCam& cam, fe_track_data& td, WarpSmem& sm, int
       if (HORIZ) {
         if (gxx < 1.1920928955078125e-07f) {
           if (lane == 0) td.track_status = 0;
-          return;
+          return differs;
         }
         det_rcp = __frcp_rn(gxx);  // correctly rounded: equals __fdiv_rn(1.f, gxx)
       } else {
         const float det = __fmaf_rn(gxx, gyy, -__fmul_rn(gxy, gxy));
         if (det < 1.1920928955078125e-07f) {
           if (lane == 0) td.track_status = 0;
-          return;
+          return differs;
         }
         det_rcp = __frcp_rn(det);  // correctly rounded: equals __fdiv_rn(1.f, det)
       }
@@ -279,6 +282,7 @@ __device__ void track_one(const LkCam& cam, fe_track_data& td, WarpSmem& sm, int
         const float d1d2 = __fmul_rn(d1, d2);
         const float ncc = d1d2 < 1.1920928955078125e-07f ? 0.f : __fmul_rn(d12, __frsqrt_rn(d1d2));
         conv = ncc > ncc_thr;
+        if (MODE == kModeRetrack) differs |= conv != (ncc > ncc_other);
       }
       if (MODE == kModeUnrolled && rec && lane == 0 && conv) rec->flags[level] |= 2;
       if (!conv && level > 0) {
@@ -378,6 +382,7 @@ __device__ void track_one(const LkCam& cam, fe_track_data& td, WarpSmem& sm, int
     }
     td.track_status = conv ? 1 : 0;
   }
+  return differs;
 }
 
 }  // namespace lk
