@@ -203,7 +203,9 @@ int plan_pyramid(const void* src, int64_t src_pitch, bool u8, const fe_pyramid& 
     if (!g) {
       plan[stage].emplace_back();
       g = &plan[stage].back();
-      memset(&g->batch, 0, sizeof(g->batch));
+      // (the jobs are written whole as they are added)
+      g->batch.njobs = g->batch.wait_limit = 0;
+      g->batch.status = g->batch.queue = nullptr;
       g->u8 = kind_u8;
       g->nl = nl;
       g->tail = has_tail;
@@ -653,7 +655,7 @@ int fe_select(fe_context* ctx, const fe_pyramid* pyr, int border_top, int border
   }
   cudaStream_t st = (cudaStream_t)stream;
   FE_CUDA(cudaMemsetAsync(s.mem, 0, s.zero_bytes, st));
-  static thread_local fe::SelectBatch b;  // large: keep off the stack
+  fe::SelectOne b;
   memset(&b, 0, sizeof(b));
   b.ncams = 1;
   b.debug = ctx->debug ? 1 : 0;
@@ -1570,7 +1572,7 @@ int fe_batch_run_plain(fe_batch* b, fe_stream stream) {
       if (rc) return rc;
       SelectScratch& s = ctx->sel;
       FE_CUDA(cudaMemsetAsync(s.mem, 0, s.zero_bytes, st));
-      static thread_local fe::SelectBatch sb;
+      fe::SelectOne sb;
       memset(&sb, 0, sizeof(sb));
       sb.ncams = 1;
       fe::SelectCam& sc = sb.cam[0];

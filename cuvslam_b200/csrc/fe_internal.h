@@ -41,15 +41,18 @@ constexpr int kMaxStageJobs = 48;  // jobs per launch (the job table is a kernel
 // Default iteration limit of the levels 0-2 kernel's bounded waits (a few hundred ms at most).
 constexpr int kDefaultWaitLimit = 1 << 22;
 
-struct StageBatch {
+template <int N>
+struct StageBatchT {
   int njobs;
   int wait_limit;           // iterations of a bounded wait before it gives up (0: at once)
   int* status;              // device flags: bit 0 = a TMA wait ran out (tile skipped), bit 1 = a
                             // deeper-level item's wait ran out (item skipped)
   int* queue;               // levels 0-2 kernel with deeper-level items: [0] next item, [1] CTAs
                             // finished (zero between launches), or nullptr: item = blockIdx.x
-  StageJob job[kMaxStageJobs];
+  StageJob job[N];
 };
+using StageBatch = StageBatchT<kMaxStageJobs>;
+using StageOne = StageBatchT<1>;  // launches of one job: a smaller kernel parameter
 static_assert(sizeof(StageBatch) <= 32000, "stage job table exceeds the kernel parameter limit");
 
 // kt: the generic stages' deepest-level tile (8 or 16), plus kL012Three to run the levels 0-2 kernel
@@ -116,14 +119,19 @@ struct SelectCam {
                                  // are then staged by TMA
 };
 
-struct SelectBatch {
+// The table of a launch is a kernel parameter, copied by every launch: single-camera launches take a
+// table of one (each of a selection's launches costs 2 us less on the host than with 17 KB).
+template <int N>
+struct SelectBatchT {
   int ncams;
   int debug;
   int* status;     // device flags (bit 2: a response tile's TMA staging did not arrive; the tile
                    // is skipped), or null
   int wait_limit;  // iterations of that bounded wait
-  SelectCam cam[kMaxCams];
+  SelectCam cam[N];
 };
+using SelectBatch = SelectBatchT<kMaxCams>;
+using SelectOne = SelectBatchT<1>;
 
 constexpr int kMaxSelectKeys = 16384;  // shared-memory sort capacity of the selection kernels
 // The [gx, gy] tensor maps of a camera's level-0 gradient planes with the response tile's gradient
@@ -135,6 +143,7 @@ cudaError_t select_init();
 // single-camera selection (burn before the response tiles; maps only when b.debug)
 cudaError_t launch_select(const SelectBatch& b, int total_tiles, int bin_key_cap, int final_key_cap,
                           cudaStream_t s);
+cudaError_t launch_select(const SelectOne& b, int total_tiles, int bin_key_cap, int final_key_cap, cudaStream_t s);
 // batched selection in two parts: the response tiles (no dependency on tracking; writes the resp and
 // nms maps) and, after tracking, the burn, the burned cells, quotas and order
 cudaError_t launch_select_response(const SelectBatch& b, int total_tiles, cudaStream_t s);

@@ -506,7 +506,8 @@ __device__ void rest_item(const Level* tail, int n, float* sm) {
 
 // Thread 0 waits (at most batch.wait_limit polls) until *ctr >= target; false (and status bit 1)
 // when the wait ran out.
-__device__ bool wait_count(const StageBatch& batch, int* ctr, int target) {
+template <typename Batch>
+__device__ bool wait_count(const Batch& batch, int* ctr, int target) {
   __shared__ int s_ok;
   if (threadIdx.x == 0) {
     int ok = 0;
@@ -528,8 +529,8 @@ __device__ bool wait_count(const StageBatch& batch, int* ctr, int target) {
 // Deeper-level item idx of job J.  J.done: [0] tiles finished, [1] phase-3 bands, [2] phase-4
 // bands; the launch's last CTA returns them to zero for the next launch (not the rest item: if one
 // of its waits gave up, tiles and bands may still be counting).
-template <int NT>
-__device__ void deep_item(const StageBatch& batch, const StageJob& J, int idx, float* sm) {
+template <int NT, typename Batch>
+__device__ void deep_item(const Batch& batch, const StageJob& J, int idx, float* sm) {
   int* ctr = J.done;
   const int ntiles = J.tiles_x * J.tiles_y;
   const int nb0 = J.deep_bands[0], nb1 = J.deep_bands[1];
@@ -674,7 +675,8 @@ __device__ __forceinline__ void levels12_outputs(const Level& L1, const Level& L
 
 // Tile t of job: levels 0-2, and when the launch computes the deeper levels, level 3's image core
 // (after which the tile counts itself complete in job.done[0]).
-__device__ __forceinline__ void l012_tile(const StageBatch& batch, const StageJob& job, int t, unsigned char* sm) {
+template <typename Batch>
+__device__ __forceinline__ void l012_tile(const Batch& batch, const StageJob& job, int t, unsigned char* sm) {
   uint8_t* B0 = sm;
   float* B1 = reinterpret_cast<float*>(sm + kOffB1);
   float* B2 = reinterpret_cast<float*>(sm + kOffB2);
@@ -967,8 +969,8 @@ __device__ __forceinline__ void l012_tile(const StageBatch& batch, const StageJo
 }
 
 // MINB: CTAs resident per SM the registers are budgeted for (2, or 3 with fewer registers).
-template <int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) pyramid_l012_kernel(const __grid_constant__ StageBatch batch) {
+template <int MINB, typename Batch>
+__global__ void __launch_bounds__(kThreads, MINB) pyramid_l012_kernel(const __grid_constant__ Batch batch) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ int s_q;
   const int tid = threadIdx.x;
@@ -1067,7 +1069,8 @@ __device__ __forceinline__ void down_pair(Load load, float2 (&acc)[ROWS]) {
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 4) pyramid_lead_kernel(const __grid_constant__ StageBatch batch) {
+template <typename Batch>
+__global__ void __launch_bounds__(kThreads, 4) pyramid_lead_kernel(const __grid_constant__ Batch batch) {
   extern __shared__ __align__(128) unsigned char sm[];
   constexpr int kS1 = G::kS1, kS1S = G::kS1S, kS2 = G::kS2, kS2S = G::kS2S;
   float* B0 = reinterpret_cast<float*>(sm);
@@ -1307,8 +1310,9 @@ __global__ void __launch_bounds__(kThreads, 4) pyramid_lead_kernel(const __grid_
 // levels are read back through L2 (cp.async.cg, __ldcg), where the other CTAs' stores are.
 constexpr int kDeepCtas = 8, kDeepThreads = 512, kDeepFloats = 12 * 1024;
 
+template <typename Batch>
 __global__ void __cluster_dims__(kDeepCtas, 1, 1) __launch_bounds__(kDeepThreads)
-    pyramid_deep_kernel(const __grid_constant__ StageBatch batch) {
+    pyramid_deep_kernel(const __grid_constant__ Batch batch) {
   extern __shared__ __align__(16) float dsm[];
   const StageJob& J = batch.job[blockIdx.x / kDeepCtas];
   const int rank = blockIdx.x % kDeepCtas;
@@ -1565,20 +1569,49 @@ bool encode_frame_tmap(StageJob& job) {
   return true;
 }
 
+namespace {
+template <typename Batch>
+cudaError_t set_l012_attrs() {
+  cudaError_t e;
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if ((e = cudaFuncSetAttribute(l012::pyramid_l012_kernel<2, Batch>, attr, l012::kSmemBox)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(l012::pyramid_l012_kernel<3, Batch>, attr, l012::kSmemBox)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(lead::pyramid_lead_kernel<Batch>, attr, lead::kSmem)) != cudaSuccess) return e;
+  return cudaFuncSetAttribute(lead::pyramid_deep_kernel<Batch>, attr, lead::kDeepFloats * 4);
+}
+
+StageOne one_job(const StageBatch& b) {
+  StageOne o;
+  o.njobs = b.njobs;
+  o.wait_limit = b.wait_limit;
+  o.status = b.status;
+  o.queue = b.queue;
+  o.job[0] = b.job[0];
+  return o;
+}
+
+template <typename Batch>
+cudaError_t launch_l012(const Batch& b, int tiles, int kt, int smem, cudaStream_t s) {
+  if (kt & kL012Three)
+    l012::pyramid_l012_kernel<3, Batch><<<tiles, l012::kThreads, smem, s>>>(b);
+  else
+    l012::pyramid_l012_kernel<2, Batch><<<tiles, l012::kThreads, smem, s>>>(b);
+  return cudaGetLastError();
+}
+
+template <typename Batch>
+cudaError_t launch_lead(const Batch& b, int tiles, bool tail, cudaStream_t s) {
+  lead::pyramid_lead_kernel<Batch><<<tiles, lead::kThreads, lead::kSmem, s>>>(b);
+  if (tail)
+    lead::pyramid_deep_kernel<Batch><<<b.njobs * lead::kDeepCtas, lead::kDeepThreads, lead::kDeepFloats * 4, s>>>(b);
+  return cudaGetLastError();
+}
+}  // namespace
+
 cudaError_t pyramid_init() {
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(l012::pyramid_l012_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                l012::kSmemBox)) != cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(l012::pyramid_l012_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                l012::kSmemBox)) != cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(lead::pyramid_lead_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                lead::kSmem)) != cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(lead::pyramid_deep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                lead::kDeepFloats * 4)) != cudaSuccess)
-    return e;
+  if ((e = set_l012_attrs<StageBatch>()) != cudaSuccess) return e;
+  if ((e = set_l012_attrs<StageOne>()) != cudaSuccess) return e;
   if ((e = set_stage_attrs<8>()) != cudaSuccess) return e;
   return set_stage_attrs<16>();
 }
@@ -1597,10 +1630,7 @@ cudaError_t launch_input_stage(const uint8_t* src, int64_t src_pitch, int channe
 
 cudaError_t launch_pyramid_lead(const StageBatch& b, int tiles, bool tail, cudaStream_t s) {
   if (tiles <= 0) return cudaSuccess;
-  lead::pyramid_lead_kernel<<<tiles, lead::kThreads, lead::kSmem, s>>>(b);
-  if (tail)
-    lead::pyramid_deep_kernel<<<b.njobs * lead::kDeepCtas, lead::kDeepThreads, lead::kDeepFloats * 4, s>>>(b);
-  return cudaGetLastError();
+  return b.njobs == 1 ? launch_lead(one_job(b), tiles, tail, s) : launch_lead(b, tiles, tail, s);
 }
 
 cudaError_t launch_pyramid_stage(const StageBatch& b, int tiles, bool u8, int nl, int kt, bool tail, cudaStream_t s) {
@@ -1613,11 +1643,7 @@ cudaError_t launch_pyramid_stage(const StageBatch& b, int tiles, bool u8, int nl
         bool box = false;
         for (int j = 0; j < b.njobs; ++j) box = box || b.job[j].box3;
         const int smem = box ? l012::kSmemBox : l012::kSmem;
-        if (kt & kL012Three)
-          l012::pyramid_l012_kernel<3><<<tiles, l012::kThreads, smem, s>>>(b);
-        else
-          l012::pyramid_l012_kernel<2><<<tiles, l012::kThreads, smem, s>>>(b);
-        return cudaGetLastError();
+        return b.njobs == 1 ? launch_l012(one_job(b), tiles, kt, smem, s) : launch_l012(b, tiles, kt, smem, s);
     }
   }
   switch (nl) {

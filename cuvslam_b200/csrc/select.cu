@@ -95,7 +95,8 @@ __device__ __forceinline__ void count_bin(const SelectCam& c, float x, float y, 
 // than `cells` of them burn, so this serves every camera with no more features than cells.  Spread over
 // the device it takes 2.2 us for 600 features and 6 us for 32 cameras of 300-3000 (one block per camera that ranked them and burned nine rows
 // a thread took 6 us for 600 features and 20 us for 32 cameras of 300-3000).
-__global__ void __launch_bounds__(288) alive_kernel(const __grid_constant__ SelectBatch b) {
+template <typename Batch>
+__global__ void __launch_bounds__(288) alive_kernel(const __grid_constant__ Batch b) {
   const SelectCam& c = b.cam[blockIdx.y];
   __shared__ int bin_cnt[64];
   __shared__ int s_alive;
@@ -119,7 +120,8 @@ __global__ void __launch_bounds__(288) alive_kernel(const __grid_constant__ Sele
 }
 
 // One block per camera, features ranked in input order: cameras with more features than cells.
-__global__ void alive_ranked_kernel(const __grid_constant__ SelectBatch b) {
+template <typename Batch>
+__global__ void alive_ranked_kernel(const __grid_constant__ Batch b) {
   const SelectCam& c = b.cam[blockIdx.x];
   __shared__ int warp_counts[32];
   __shared__ int base;
@@ -205,8 +207,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t phase, 
 }
 
 
-template <bool kSplit>
-__global__ void __launch_bounds__(tile::kThreads) tile_kernel(const __grid_constant__ SelectBatch b) {
+template <bool kSplit, typename Batch>
+__global__ void __launch_bounds__(tile::kThreads) tile_kernel(const __grid_constant__ Batch b) {
   using namespace tile;
   extern __shared__ __align__(128) unsigned char tsm[];
   float* hxx = reinterpret_cast<float*>(tsm + kOffH);
@@ -722,7 +724,8 @@ __device__ uint64_t block_select_kth(const uint64_t* keys, int n, int k) {
   return s_prefix;
 }
 
-__global__ void __launch_bounds__(256) bin_kernel(const __grid_constant__ SelectBatch b, int key_cap) {
+template <typename Batch>
+__global__ void __launch_bounds__(256) bin_kernel(const __grid_constant__ Batch b, int key_cap) {
   extern __shared__ uint64_t keys[];
   __shared__ int count;
   const SelectCam& c = b.cam[blockIdx.y];
@@ -781,7 +784,8 @@ __global__ void __launch_bounds__(256) bin_kernel(const __grid_constant__ Select
 // bitonic sort per camera).
 constexpr int kRankKeys = 32, kRankChunk = 2048;
 
-__global__ void __launch_bounds__(kRankKeys * 8) final_kernel(const __grid_constant__ SelectBatch b, int key_cap) {
+template <typename Batch>
+__global__ void __launch_bounds__(kRankKeys * 8) final_kernel(const __grid_constant__ Batch b, int key_cap) {
   __shared__ uint64_t keys[kRankChunk];
   const SelectCam& c = b.cam[blockIdx.y];
   const int n = min(min(c.stats[2], c.q_cap), key_cap), out = min(n, wanted_features(c));
@@ -820,22 +824,32 @@ bool encode_select_grad_tmaps(CUtensorMap* maps, const float* gx, const float* g
 int select_tile_w() { return tile::TW; }
 int select_tile_h() { return tile::TH; }
 
-cudaError_t select_init() {
-  cudaError_t e = cudaFuncSetAttribute(tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile::kSmem);
+namespace {
+template <typename Batch>
+cudaError_t set_attrs() {
+  cudaError_t e = cudaFuncSetAttribute(tile_kernel<false, Batch>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile::kSmem);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile::kSmem);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(bin_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(bin_kernel<Batch>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(sizeof(uint64_t) * kMaxSelectKeys));
+}
+}  // namespace
+
+cudaError_t select_init() {
+  cudaError_t e = cudaFuncSetAttribute(tile_kernel<true, SelectBatch>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       tile::kSmem);
+  if (e == cudaSuccess) e = set_attrs<SelectBatch>();
+  if (e == cudaSuccess) e = set_attrs<SelectOne>();
+  return e;
 }
 
 cudaError_t launch_select_response(const SelectBatch& b, int total_tiles, cudaStream_t s) {
-  tile_kernel<true><<<total_tiles, tile::kThreads, tile::kSmem, s>>>(b);
+  tile_kernel<true, SelectBatch><<<total_tiles, tile::kThreads, tile::kSmem, s>>>(b);
   return cudaGetLastError();
 }
 
 namespace {
-cudaError_t launch_bins_final(const SelectBatch& b, int bin_key_cap, int final_key_cap, cudaStream_t s) {
+template <typename Batch>
+cudaError_t launch_bins_final(const Batch& b, int bin_key_cap, int final_key_cap, cudaStream_t s) {
   bin_kernel<<<dim3(64, b.ncams), 256, sizeof(uint64_t) * bin_key_cap, s>>>(b, bin_key_cap);
   int q_cap = 1;
   for (int i = 0; i < b.ncams; ++i) q_cap = max(q_cap, b.cam[i].q_cap);
@@ -845,7 +859,8 @@ cudaError_t launch_bins_final(const SelectBatch& b, int bin_key_cap, int final_k
 }
 
 // The alive features of every camera; nothing to do without any (the counters are zero).
-void launch_alive(const SelectBatch& b, cudaStream_t s) {
+template <typename Batch>
+void launch_alive(const Batch& b, cudaStream_t s) {
   int most = 0;
   bool ranked = false;
   for (int i = 0; i < b.ncams; ++i) {
@@ -869,12 +884,23 @@ cudaError_t launch_select_rest(const SelectBatch& b, int touched_words, int bin_
   return launch_bins_final(b, bin_key_cap, final_key_cap, s);
 }
 
-cudaError_t launch_select(const SelectBatch& b, int total_tiles, int bin_key_cap, int final_key_cap,
-                          cudaStream_t s) {
+namespace {
+template <typename Batch>
+cudaError_t launch_burned(const Batch& b, int total_tiles, int bin_key_cap, int final_key_cap, cudaStream_t s) {
   if (bin_key_cap > kMaxSelectKeys || final_key_cap > kMaxSelectKeys) return cudaErrorInvalidValue;
   launch_alive(b, s);
-  tile_kernel<false><<<total_tiles, tile::kThreads, tile::kSmem, s>>>(b);
+  tile_kernel<false, Batch><<<total_tiles, tile::kThreads, tile::kSmem, s>>>(b);
   return launch_bins_final(b, bin_key_cap, final_key_cap, s);
+}
+}  // namespace
+
+cudaError_t launch_select(const SelectBatch& b, int total_tiles, int bin_key_cap, int final_key_cap,
+                          cudaStream_t s) {
+  return launch_burned(b, total_tiles, bin_key_cap, final_key_cap, s);
+}
+
+cudaError_t launch_select(const SelectOne& b, int total_tiles, int bin_key_cap, int final_key_cap, cudaStream_t s) {
+  return launch_burned(b, total_tiles, bin_key_cap, final_key_cap, s);
 }
 
 }  // namespace fe

@@ -138,7 +138,7 @@ extern "C" FE_API int fe_select_noalloc(const fe_pyramid* pyr, int border_top, i
   // the array keeps the previous call's contents: clear the counters and the burn mask
   if (cudaMemsetAsync(s, 0, L.zero_end, st) != cudaSuccess) return FE_ERR_CUDA;
 
-  static thread_local fe::SelectBatch b;
+  fe::SelectOne b;
   memset(&b, 0, sizeof(b));
   b.ncams = 1;
   fe::SelectCam& c = b.cam[0];

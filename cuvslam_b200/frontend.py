@@ -26,8 +26,10 @@ DEFAULT_LK_SAMPLING = _lib.FE_SAMPLE_HARDWARE
 
 
 def _stream_handle(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    """The stream's handle, or the current device's current stream's (without a Stream object made for it)."""
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _ptr(t):
@@ -163,11 +165,16 @@ def tracks_to_device(tracks, device="cuda"):
     """TRACK_DTYPE records -> (n, 80) uint8 CUDA tensor (the TrackData array the kernels update,
     cuda_kernels.h:76-87)."""
     arr = np.ascontiguousarray(tracks, dtype=TRACK_DTYPE)
-    return torch.from_numpy(arr.view(np.uint8).reshape(len(arr), 80).copy()).to(device)
+    raw = arr.view(np.uint8).reshape(len(arr), 80)
+    if not raw.flags.writeable or torch.device(device).type == "cpu":
+        raw = raw.copy()  # (the copy to a device is the tensor's own memory)
+    return torch.from_numpy(raw).to(device)
 
 
 def tracks_from_device(t):
-    return t.cpu().numpy().reshape(-1).view(TRACK_DTYPE).copy()
+    # a device tensor's host copy is the records' own memory (copying a structured array goes field by field)
+    recs = t.cpu().numpy().reshape(-1).view(TRACK_DTYPE)
+    return recs if t.is_cuda else recs.copy()
 
 
 class LKFeatureTracker:
@@ -274,7 +281,7 @@ class Selection:
                      num_desired, stream=None):
         """Enqueues selection; returns (xy (num_desired, 2) tensor, count (1,) int32 tensor)."""
         out = torch.empty((max(int(num_desired), 1), 2), dtype=torch.float32, device=self.ctx.device)
-        count = torch.zeros(1, dtype=torch.int32, device=self.ctx.device)
+        count = torch.empty(1, dtype=torch.int32, device=self.ctx.device)  # written by every selection
         alive = None
         n_alive = 0
         if alive_features is not None and len(alive_features) > 0:
@@ -296,8 +303,9 @@ class Selection:
         """Blocking form with the reference's signature: returns the new features as an (k, 2) tensor."""
         out, count = self.select_async(pyramid, border_top, border_bottom, border_left, border_right, input_mask,
                                        alive_features, num_desired_new_features, stream)
-        (stream or torch.cuda.current_stream()).synchronize()
-        return out[: int(count.item())]
+        if stream is not None:
+            stream.synchronize()
+        return out[: int(count.item())]  # (item() waits for the current stream)
 
     def debug_maps(self, width, height):
         """(response, nms) maps of the last selection as (height, width) float32 CUDA tensors; the
