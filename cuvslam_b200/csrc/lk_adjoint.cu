@@ -51,16 +51,22 @@ struct AdjSmem {
   WarpSmem win;               // staging windows, as the forward
   float acc[32 * 32];         // current-image record
   float prec[3][kRP * kRP];   // previous-image records
-  float coef[3][81];          // tap coefficients (serial scatter)
-  int cb[9], rb[9];           // column / row texel index (serial scatter)
+  float coef[3][81];          // tap coefficients (scatter by pixel)
+  int cb[9], rb[9];           // column / row texel index (scatter by pixel)
   float cf[9], rf[9];         // column / row fraction
+  unsigned cm[32], rm[32];    // tap columns / rows that reach a record column / row: left or upper texel in
+                              // bits 0-8, right or lower in bits 16-24
 };
 
 // Adds the transposed bilinear taps of NP coefficient sets (tap f = lane + 32 e) into shared-memory
 // records dst[p] (row stride rs, origin (rx0, ry0) in level texels).  Texel indices are clamped to
 // the W x H level as the forward's staged windows clamp them.  When all taps share their fractions
-// and none clamps, four conflict-free passes (one per bilinear corner) add the taps; otherwise lane 0
-// adds every tap in order.  Both are deterministic.
+// and none clamps, four conflict-free passes (one per bilinear corner) add the taps.  Otherwise (a
+// fraction rounds differently where the coordinates cross a power of two, which most patches of the
+// coarse levels do) each lane takes record pixels and adds the taps that reach them in tap order, each
+// tap's corners in order: the sums of a serial pass over the taps, which took one lane some 20 000 cycles a
+// step (the unrolled backward of 8 x 4096 tracks at 1280x720 spent half its adjoint kernel there).
+// Both are deterministic.
 template <int NP>
 __device__ void scatter_taps(float* const (&dst)[NP], int rs, int rx0, int ry0, const TapSet& ts,
                              const float (&c)[NP][kNE], const bool (&valid)[kNE], const int (&ix)[kNE],
@@ -100,22 +106,46 @@ __device__ void scatter_taps(float* const (&dst)[NP], int rs, int rx0, int ry0, 
     sm.rf[lane - 16] = ts.fr;
   }
   __syncwarp();
-  if (lane == 0) {
-    for (int f = 0; f < 81; ++f) {
-      const int i = f % 9, j = f / 9;
-      const float fx = sm.cf[i], fy = sm.rf[j];
-      const float gx = __fsub_rn(1.f, fx), gy = __fsub_rn(1.f, fy);
-      const int x0 = min(max(sm.cb[i], 0), W - 1) - rx0, x1 = min(max(sm.cb[i] + 1, 0), W - 1) - rx0;
-      const int y0 = min(max(sm.rb[j], 0), H - 1) - ry0, y1 = min(max(sm.rb[j] + 1, 0), H - 1) - ry0;
+  unsigned cm = 0, rm = 0;
 #pragma unroll
-      for (int q = 0; q < NP; ++q) {
-        const float v = sm.coef[q][f];
-        dst[q][y0 * rs + x0] = __fmaf_rn(__fmul_rn(gx, gy), v, dst[q][y0 * rs + x0]);
-        dst[q][y0 * rs + x1] = __fmaf_rn(__fmul_rn(fx, gy), v, dst[q][y0 * rs + x1]);
-        dst[q][y1 * rs + x0] = __fmaf_rn(__fmul_rn(gx, fy), v, dst[q][y1 * rs + x0]);
-        dst[q][y1 * rs + x1] = __fmaf_rn(__fmul_rn(fx, fy), v, dst[q][y1 * rs + x1]);
+  for (int i = 0; i < 9; ++i) {
+    const int cb = sm.cb[i], rb = sm.rb[i];
+    if (min(max(cb, 0), W - 1) - rx0 == lane) cm |= 1u << i;
+    if (min(max(cb + 1, 0), W - 1) - rx0 == lane) cm |= 1u << (16 + i);
+    if (min(max(rb, 0), H - 1) - ry0 == lane) rm |= 1u << i;
+    if (min(max(rb + 1, 0), H - 1) - ry0 == lane) rm |= 1u << (16 + i);
+  }
+  sm.cm[lane] = cm;
+  sm.rm[lane] = rm;
+  const unsigned cols = __ballot_sync(kFull, cm != 0), rows = __ballot_sync(kFull, rm != 0);
+  const int xlo = __ffs(cols) - 1, nx = 32 - __clz(cols) - xlo, ylo = __ffs(rows) - 1, ny = 32 - __clz(rows) - ylo;
+  __syncwarp();
+  for (int k = lane; k < nx * ny; k += 32) {
+    const int y = ylo + k / nx, x = xlo + k % nx;
+    const unsigned cx = sm.cm[x], ry = sm.rm[y];
+    float acc[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) acc[q] = dst[q][y * rs + x];
+    for (unsigned rj = (ry | ry >> 16) & 0x1ffu; rj; rj &= rj - 1) {
+      const int j = __ffs(rj) - 1;
+      const float fy = sm.rf[j], gy = __fsub_rn(1.f, fy);
+      const bool y0 = (ry >> j) & 1u, y1 = (ry >> (16 + j)) & 1u;
+      for (unsigned ci = (cx | cx >> 16) & 0x1ffu; ci; ci &= ci - 1) {
+        const int i = __ffs(ci) - 1;
+        const float fx = sm.cf[i], gx = __fsub_rn(1.f, fx);
+        const bool x0 = (cx >> i) & 1u, x1 = (cx >> (16 + i)) & 1u;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          const float v = sm.coef[q][9 * j + i];
+          if (x0 && y0) acc[q] = __fmaf_rn(__fmul_rn(gx, gy), v, acc[q]);
+          if (x1 && y0) acc[q] = __fmaf_rn(__fmul_rn(fx, gy), v, acc[q]);
+          if (x0 && y1) acc[q] = __fmaf_rn(__fmul_rn(gx, fy), v, acc[q]);
+          if (x1 && y1) acc[q] = __fmaf_rn(__fmul_rn(fx, fy), v, acc[q]);
+        }
       }
     }
+#pragma unroll
+    for (int q = 0; q < NP; ++q) dst[q][y * rs + x] = acc[q];
   }
   __syncwarp();
 }
