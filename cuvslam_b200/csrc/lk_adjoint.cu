@@ -698,8 +698,8 @@ __global__ void bin_kernel(const __grid_constant__ AdjGather G) {
     }
 }
 
-// Exclusive prefix sum of the per-tile counts (one CTA, four tiles per thread per pass); clears the
-// fill cursors and lists the tiles with more than kWarpList records.
+// Exclusive prefix sum of the per-tile counts (one CTA, sixteen tiles per thread per pass: a pass is a
+// chain of loads, shuffles and barriers, so fewer and wider ones are faster); clears the fill cursors and lists the tiles with more than kWarpList records.
 __global__ void __launch_bounds__(1024) scan_kernel(const __grid_constant__ AdjGather G) {
   __shared__ int warp_tot[32];
   __shared__ int carry;
@@ -709,15 +709,35 @@ __global__ void __launch_bounds__(1024) scan_kernel(const __grid_constant__ AdjG
     *G.long_count = 0;
   }
   __syncthreads();
-  for (int base = 0; base < G.total_tiles; base += 4096) {
-    const int t0 = base + 4 * tid;
-    int v[4];
+  constexpr int kPer = 16;
+  for (int base = 0; base < G.total_tiles; base += 1024 * kPer) {
+    const int t0 = base + kPer * tid;
+    int v[kPer], mine = 0;
+    if (t0 + kPer <= G.total_tiles) {  // (the counts start 16-byte aligned)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      v[k] = t0 + k < G.total_tiles ? G.count[t0 + k] : 0;
-      if (v[k] > kWarpList) G.long_tiles[atomicAdd(G.long_count, 1)] = t0 + k;  // processing order is free
+      for (int k = 0; k < kPer; k += 4) {
+        const int4 q = *reinterpret_cast<const int4*>(G.count + t0 + k);
+        v[k] = q.x;
+        v[k + 1] = q.y;
+        v[k + 2] = q.z;
+        v[k + 3] = q.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) v[k] = t0 + k < G.total_tiles ? G.count[t0 + k] : 0;
     }
-    const int mine = v[0] + v[1] + v[2] + v[3];
+    int nlong = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      nlong += v[k] > kWarpList ? 1 : 0;
+      mine += v[k];
+    }
+    if (nlong) {
+      int at = atomicAdd(G.long_count, nlong);  // processing order is free
+#pragma unroll
+      for (int k = 0; k < kPer; ++k)
+        if (v[k] > kWarpList) G.long_tiles[at++] = t0 + k;
+    }
     int x = mine;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -737,13 +757,23 @@ __global__ void __launch_bounds__(1024) scan_kernel(const __grid_constant__ AdjG
     }
     __syncthreads();
     int before = carry + (wid > 0 ? warp_tot[wid - 1] : 0) + x - mine;
+    if (t0 + kPer <= G.total_tiles) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (t0 + k < G.total_tiles) {
-        G.off[t0 + k] = before;
-        G.cursor[t0 + k] = 0;
+      for (int k = 0; k < kPer; k += 4) {
+        const int4 q = make_int4(before, before + v[k], before + v[k] + v[k + 1], before + v[k] + v[k + 1] + v[k + 2]);
+        *reinterpret_cast<int4*>(G.off + t0 + k) = q;
+        *reinterpret_cast<int4*>(G.cursor + t0 + k) = make_int4(0, 0, 0, 0);
+        before = q.w + v[k + 3];
       }
-      before += v[k];
+    } else {
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        if (t0 + k < G.total_tiles) {
+          G.off[t0 + k] = before;
+          G.cursor[t0 + k] = 0;
+        }
+        before += v[k];
+      }
     }
     __syncthreads();
     if (tid == 0) carry += warp_tot[31];
@@ -772,34 +802,53 @@ __device__ __forceinline__ const AdjPlane& tile_plane(const AdjGather& G, int t)
   return G.planes[lo];
 }
 
-// One warp adds records to its 32x32 tile at (X0, Y0): lane = column X0 + lane, acc[r] = row Y0 + r.
-// `key` is this lane's record slot (lanes 0..m-1 hold m records, in the order they are added).
-__device__ __forceinline__ void warp_add_records(const AdjGather& G, int key, int m, int X0, int Y0, float (&acc)[kTile],
+// One warp adds records to its 32x32 tile at (X0, Y0), `acc` in shared memory (row stride kTile).
+// `key` is this lane's record slot (lanes 0..m-1 hold m records, in the order they are added: a pixel gets
+// one value per record, so the rows of a record are added side by side, two at a time where the record
+// is at most 16 wide).  The adds of a record are bound by issue, not by memory: with a column per lane and
+// the tile's 32 rows in registers every record cost its warp all 32 rows, whatever it covers.
+__device__ __forceinline__ void warp_add_records(const AdjGather& G, int key, int m, int X0, int Y0, float* acc,
                                                  int lane) {
   const int4 mine = lane < m ? G.hdr[key] : make_int4(0, 0, 0, 0);
-  const int X = X0 + lane;
+  // the record's columns and rows inside the tile, and its value at the first of them
+  const int x0 = max(mine.x - X0, 0), x1 = min(mine.x + mine.z - X0, kTile);
+  const int y0 = max(mine.y - Y0, 0), y1 = min(mine.y + mine.w - Y0, kTile);
+  int S = 0;
+  const float* d = nullptr;
   if (lane < m) {
+    d = record_data(G, key, S) + (y0 + Y0 - mine.y) * S + (x0 + X0 - mine.x);
     // every record of the group is requested into L2 up front (lane r: record r's rows inside the
     // tile), so that the in-order adds below wait on L2 rather than on DRAM
-    int S;
-    const float* d = record_data(G, key, S) + max(0, X0 - mine.x);
-    const int r1 = min(mine.w, Y0 + kTile - mine.y);
-    for (int row = max(0, Y0 - mine.y); row < r1; ++row)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(d + (size_t)row * S));
+    for (int row = 0; row < y1 - y0; ++row) asm volatile("prefetch.global.L2 [%0];" ::"l"(d + (size_t)row * S));
   }
+  const int box = x0 | (x1 - x0) << 8 | y0 << 16 | (y1 - y0) << 24;  // each part in 0..32
   for (int r = 0; r < m; ++r) {
-    const int k = __shfl_sync(kFull, key, r);
-    const int hx = __shfl_sync(kFull, mine.x, r), hy = __shfl_sync(kFull, mine.y, r);
-    const int hz = __shfl_sync(kFull, mine.z, r), hw = __shfl_sync(kFull, mine.w, r);
-    if (X < hx || X >= hx + hz || hy >= Y0 + kTile || hy + hw <= Y0) continue;
-    int S;
-    const float* d = record_data(G, k, S) + (X - hx);
-#pragma unroll
-    for (int row = 0; row < kTile; ++row) {
-      const int dy = Y0 + row - hy;
-      if (dy >= 0 && dy < hw) acc[row] += d[dy * S];
+    const int b = __shfl_sync(kFull, box, r), s = __shfl_sync(kFull, S, r);
+    const float* q = reinterpret_cast<const float*>(__shfl_sync(kFull, (unsigned long long)d, r));
+    const int bx = b & 255, bw = (b >> 8) & 255, by = (b >> 16) & 255, bh = (b >> 24) & 255;
+    if (bw <= 16) {
+      const int c = lane & 15, h = lane >> 4;
+      if (c < bw) {
+        float* a = acc + (by + h) * kTile + bx + c;
+        q += h * s + c;
+#pragma unroll 8
+        for (int row = h; row < bh; row += 2, a += 2 * kTile, q += 2 * s) *a += __ldg(q);
+      }
+    } else if (lane < bw) {
+      float* a = acc + by * kTile + bx + lane;
+      q += lane;
+#pragma unroll 8
+      for (int row = 0; row < bh; ++row, a += kTile, q += s) *a += __ldg(q);
     }
+    __syncwarp();
   }
+}
+
+__device__ __forceinline__ void zero_tile(float* acc, int lane) {
+#pragma unroll
+  for (int r = 0; r < kTile * kTile / 128; ++r)
+    reinterpret_cast<float4*>(acc)[r * 32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncwarp();
 }
 
 // Ascending sort of one key per lane across the warp (bitonic network on shuffles).
@@ -818,8 +867,9 @@ __device__ __forceinline__ int warp_sort(int key, int lane) {
 }
 
 // Tiles with at most kWarpList records (nearly all): one warp per tile, 8 tiles per CTA; the warp
-// sorts the slots (track order) and adds the records in that order into its registers.
+// sorts the slots (track order) and adds the records in that order.
 __global__ void __launch_bounds__(kGatherThreads) gather_warp_kernel(const __grid_constant__ AdjGather G) {
+  __shared__ __align__(16) float tiles[kGatherWarps][kTile * kTile];
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * kGatherWarps + (threadIdx.x >> 5);
   if (t >= G.total_tiles) return;  // warp-uniform
@@ -828,22 +878,28 @@ __global__ void __launch_bounds__(kGatherThreads) gather_warp_kernel(const __gri
   const AdjPlane& P = tile_plane(G, t);
   const int lt = t - P.tile_begin;
   const int X0 = (lt % P.tiles_x) * kTile, Y0 = (lt / P.tiles_x) * kTile;
-  const int key = warp_sort(lane < n ? G.list[begin + lane] : INT_MAX, lane);
-  float acc[kTile];
+  float* acc = tiles[threadIdx.x >> 5];
+  zero_tile(acc, lane);
+  if (n > 0)
+    warp_add_records(G, warp_sort(lane < n ? G.list[begin + lane] : INT_MAX, lane), n, X0, Y0, acc, lane);
+  if (X0 + kTile <= P.w && Y0 + kTile <= P.h && (P.pitch & 3) == 0 && (reinterpret_cast<uintptr_t>(P.dst) & 15) == 0) {
+    float* o = P.dst + (size_t)(Y0 + (lane >> 3)) * P.pitch + X0 + 4 * (lane & 7);
 #pragma unroll
-  for (int r = 0; r < kTile; ++r) acc[r] = 0.f;
-  warp_add_records(G, key, n, X0, Y0, acc, lane);
+    for (int r = 0; r < kTile; r += 4)
+      *reinterpret_cast<float4*>(o + (size_t)r * P.pitch) = reinterpret_cast<const float4*>(acc + r * kTile)[lane];
+    return;
+  }
   const int X = X0 + lane;
   if (X < P.w) {
 #pragma unroll
     for (int r = 0; r < kTile; ++r)
-      if (Y0 + r < P.h) P.dst[(size_t)(Y0 + r) * P.pitch + X] = acc[r];
+      if (Y0 + r < P.h) P.dst[(size_t)(Y0 + r) * P.pitch + X] = acc[r * kTile + lane];
   }
 }
 
 // Tiles with more than kWarpList records (coarse levels), from the scan's list: a CTA orders the
 // tile's slots by track, warp k of 32 adds the k-th contiguous part of the sorted list (32 records at a time)
-// into its registers, and the 32 partial tiles are summed in warp order.  Each record costs its warp
+// into its own tile in shared memory, and the 32 partial tiles are summed in warp order.  Each record costs its warp
 // one memory round trip, so the records of a tile are spread over as many warps as one CTA holds.
 __global__ void __launch_bounds__(kLongThreads, 1) gather_long_kernel(const __grid_constant__ AdjGather G) {
   extern __shared__ __align__(16) unsigned char gsm[];
@@ -904,16 +960,13 @@ __global__ void __launch_bounds__(kLongThreads, 1) gather_long_kernel(const __gr
       keys[prefix[rel >> 5] + __popc(bits[rel >> 5] & ((1u << (rel & 31)) - 1u))] = key;
     }
     __syncthreads();
-    float acc[kTile];
-#pragma unroll
-    for (int r = 0; r < kTile; ++r) acc[r] = 0.f;
+    float* acc = part + wid * kTile * kTile;
+    zero_tile(acc, lane);
     const int r0 = (int)((long long)n * wid / kLongWarps), r1 = (int)((long long)n * (wid + 1) / kLongWarps);
     for (int g0 = r0; g0 < r1; g0 += 32) {
       const int m = min(32, r1 - g0);
       warp_add_records(G, lane < m ? keys[g0 + lane] : 0, m, X0, Y0, acc, lane);
     }
-#pragma unroll
-    for (int r = 0; r < kTile; ++r) part[wid * kTile * kTile + r * kTile + lane] = acc[r];
     __syncthreads();
     for (int k = tid; k < kTile * kTile; k += kLongThreads) {
       const int X = X0 + (k & (kTile - 1)), Y = Y0 + k / kTile;
@@ -929,6 +982,27 @@ __global__ void __launch_bounds__(kLongThreads, 1) gather_long_kernel(const __gr
 // ---------------------------------------------------------------- pyramid adjoint
 __device__ __forceinline__ float binom5(int k) {
   return k == 2 ? 6.f / 16.f : (k == 1 || k == 3) ? 4.f / 16.f : 1.f / 16.f;
+}
+
+// The next level's coordinates (of m) along one axis whose 5 taps read coordinate c of n, with the taps'
+// weights, in the order their contributions are added: up to three direct ones (2X - 2 + k == c, k
+// ascending), then the one that reaches c through the mirror below 0 (c = 0: X = 0 by tap 1; c = 1: X = 0
+// by tap 0), then the one through the mirror above n - 1 (virtual coordinate 2n - c - 1, read by X = m - 1
+// alone: c = n - 1 by tap 4 of an even n or tap 3 of an odd one, c = n - 2 by tap 4 of an odd n).  -1: none.
+// Straight-line code whose loads do not wait on one another: as nested loops over the taps a border pixel
+// took some 10 000 cycles, which every level's launch waited for.
+__device__ __forceinline__ void axis_sources(int c, int n, int m, int (&X)[5], float (&w)[5]) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int k = (c & 1) + 2 * j, p = (c + 2 - k) >> 1;
+    X[j] = k < 5 && p >= 0 && p < m ? p : -1;
+    w[j] = binom5(k);
+  }
+  X[3] = c <= 1 ? 0 : -1;
+  w[3] = c == 0 ? binom5(1) : binom5(0);
+  const bool odd = (n & 1) != 0;
+  X[4] = c == n - 1 || (odd && c == n - 2) ? m - 1 : -1;
+  w[4] = c == n - 1 && odd ? binom5(3) : binom5(4);
 }
 
 // Complete gradient of pixel (x, y) of one level: the summed records, the transposed 7-tap
@@ -950,47 +1024,24 @@ __device__ float adjoint_pixel(const AdjPyrJob& J, int x, int y) {
       if (yp > 2 && yp < J.h - 3) v = __fmaf_rn(dsp_tap(j), J.gy[(size_t)yp * J.gpitch + x], v);
     }
   }
-  if (J.up && x >= 2 && x <= J.w - 3 && y >= 2 && y <= J.h - 3) {
-    // interior: only unmirrored sources, 2X - 2 + k == x with k of x's parity (2 or 3 per axis)
-    for (int ky = y & 1; ky < 5; ky += 2) {
-      const int Y = (y + 2 - ky) >> 1;
-      if (Y >= J.up_h) continue;
-      const float* row = J.up + (size_t)Y * J.up_pitch;
-      const float wy = binom5(ky);
-      for (int kx = x & 1; kx < 5; kx += 2) {
-        const int X = (x + 2 - kx) >> 1;
-        if (X >= J.up_w) continue;
-        v = __fmaf_rn(__fmul_rn(wy, binom5(kx)), row[X], v);
-      }
-    }
-  } else if (J.up) {
+  if (J.up) {
     // transposed decimation: the outputs (X, Y) of the next level whose 5x5 taps read (x, y), either
     // directly (unmirrored source coordinate 2X - 2 + k == x) or through the mirror (-x-1 below 0,
     // 2n-x-1 above n-1); taps outside in both directions are skipped as the forward skips them
-    for (int a = 0; a < 3; ++a) {
-      const int yc = a == 0 ? y : a == 1 ? (y <= 1 ? -y - 1 : INT_MIN) : (y >= J.h - 2 ? 2 * J.h - y - 1 : INT_MIN);
-      if (yc == INT_MIN) continue;
-      const bool yo = yc < 0 || yc >= J.h;
-      for (int ky = 0; ky < 5; ++ky) {
-        const int vy = yc + 2 - ky;
-        if (vy & 1) continue;
-        const int Y = vy / 2;
-        if (Y < 0 || Y >= J.up_h) continue;
-        const float* row = J.up + (size_t)Y * J.up_pitch;
-        for (int b = 0; b < 3; ++b) {
-          const int xc = b == 0 ? x : b == 1 ? (x <= 1 ? -x - 1 : INT_MIN) : (x >= J.w - 2 ? 2 * J.w - x - 1 : INT_MIN);
-          if (xc == INT_MIN) continue;
-          const bool xo = xc < 0 || xc >= J.w;
-          if (xo && yo) continue;
-          for (int kx = 0; kx < 5; ++kx) {
-            const int vx = xc + 2 - kx;
-            if (vx & 1) continue;
-            const int X = vx / 2;
-            if (X < 0 || X >= J.up_w) continue;
-            v = __fmaf_rn(__fmul_rn(binom5(ky), binom5(kx)), row[X], v);
-          }
-        }
-      }
+    int X[5], Y[5];
+    float wx[5], wy[5];
+    axis_sources(x, J.w, J.up_w, X, wx);
+    axis_sources(y, J.h, J.up_h, Y, wy);
+#pragma unroll
+    for (int a = 0; a < 5; ++a) {
+      if (Y[a] < 0) continue;
+      const float* row = J.up + (size_t)Y[a] * J.up_pitch;
+      float u[5];
+#pragma unroll
+      for (int b = 0; b < 5; ++b) u[b] = X[b] >= 0 && (a < 3 || b < 3) ? row[X[b]] : 0.f;
+#pragma unroll
+      for (int b = 0; b < 5; ++b)
+        if (X[b] >= 0 && (a < 3 || b < 3)) v = __fmaf_rn(__fmul_rn(wy[a], wx[b]), u[b], v);
     }
   }
   return v;
@@ -1010,7 +1061,7 @@ __device__ __forceinline__ void load4(const float* p, float* out) {
 // rows at x .. x+3, and two or three rows of the next level's gradient from the 4-aligned column at
 // or below x/2 - 1; every pixel adds the same taps in the same order as adjoint_pixel.  Elsewhere
 // each pixel runs adjoint_pixel.
-__global__ void __launch_bounds__(256) pyramid_adjoint_kernel(const __grid_constant__ AdjPyrLevel L) {
+__global__ void __launch_bounds__(256, 5) pyramid_adjoint_kernel(const __grid_constant__ AdjPyrLevel L) {
   const AdjPyrJob& J = L.job[blockIdx.y];
   const int bx = (J.w + 127) >> 7;
   const int x = ((int)(blockIdx.x % bx) * 32 + (threadIdx.x & 31)) * 4;
@@ -1051,18 +1102,20 @@ __global__ void __launch_bounds__(256) pyramid_adjoint_kernel(const __grid_const
     }
   }
   if (J.up) {
-    // pixel x + i reads next-level columns (x + i + 2 - kx) / 2 for kx of its parity, rows likewise
-    for (int ky = y & 1; ky < 5; ky += 2) {
-      const int Y = (y + 2 - ky) >> 1;
-      float u[8];
-      const float* ur = J.up + (size_t)Y * J.up_pitch + ub;
-      load4(ur, u);
-      load4(ur + 4, u + 4);
+    // pixel x + i reads next-level columns (x + i + 2 - kx) / 2 for kx of its parity (x / 2 - 1 .. x / 2 + 2),
+    // rows likewise
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int ky = (y & 1) + 2 * j;
+      if (ky >= 5) continue;
+      const float* ur = J.up + (size_t)((y + 2 - ky) >> 1) * J.up_pitch + (x >> 1);
+      const float2 mid = *reinterpret_cast<const float2*>(ur);
+      const float u[4] = {ur[-1], mid.x, mid.y, ur[2]};
       const float wy = binom5(ky);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int kx = i & 1; kx < 5; kx += 2) v[i] = __fmaf_rn(__fmul_rn(wy, binom5(kx)), u[((x + i + 2 - kx) >> 1) - ub], v[i]);
+        for (int kx = i & 1; kx < 5; kx += 2) v[i] = __fmaf_rn(__fmul_rn(wy, binom5(kx)), u[((i + 2 - kx) >> 1) + 1], v[i]);
     }
   }
   *reinterpret_cast<float4*>(J.img + (size_t)y * J.pitch + x) = make_float4(v[0], v[1], v[2], v[3]);
