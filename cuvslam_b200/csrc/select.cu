@@ -182,7 +182,9 @@ constexpr int RW = TW + 2;                   // response region width (height TH
 constexpr int GW = TW + 10, GH = TH + 8;     // gradients loaded (two spare columns for 4-wide quads)
 constexpr int GS = 76;                       // row stride of the gradient planes (16-byte rows)
 constexpr int HS = 68;                       // row stride of the horizontal sums (>= RW, 4-aligned)
-constexpr int RS = 68;                       // row stride of the response
+constexpr int RS = 80;                       // row stride of the response (two rows of 16 columns: 32 banks)
+constexpr int NS = 72;                       // row stride of the NMS map (four rows of 8 columns: 32 banks)
+static_assert(TH * NS <= GH * HS && (TH + 2) * RS <= 2 * GH * GS, "the aliases fit");
 constexpr int kThreads = 256;
 constexpr int kOffH = 0;                                     // 3 planes [GH][HS]
 constexpr int kOffG = kOffH + 3 * GH * HS * 4;               // 2 planes [GH][GS]
@@ -293,11 +295,17 @@ __global__ void __launch_bounds__(tile::kThreads) tile_kernel(const __grid_const
   //    FP32x2 arithmetic: xx += (c_j gx) gx, xy += (c_j gx) gy, yy += (c_j gy) gy (gftt.cu:131-137)
   for (int qd = tid; qd < GH * (HS / 4); qd += kThreads) {
     const int r = qd / (HS / 4), q0 = (qd - r * (HS / 4)) * 4;
-    float2 ax[5], ay[5];
+    // (16-byte loads: their lanes' addresses are adjacent, 8-byte ones 16 bytes apart would meet in
+    // half the banks; the last two columns are not used)
+    float2 ax[6], ay[6];
 #pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      ax[m] = *reinterpret_cast<const float2*>(gxs + r * GS + q0 + 2 * m);
-      ay[m] = *reinterpret_cast<const float2*>(gys + r * GS + q0 + 2 * m);
+    for (int m = 0; m < 3; ++m) {
+      const float4 u = *reinterpret_cast<const float4*>(gxs + r * GS + q0 + 4 * m);
+      const float4 v = *reinterpret_cast<const float4*>(gys + r * GS + q0 + 4 * m);
+      ax[2 * m] = make_float2(u.x, u.y);
+      ax[2 * m + 1] = make_float2(u.z, u.w);
+      ay[2 * m] = make_float2(v.x, v.y);
+      ay[2 * m + 1] = make_float2(v.z, v.w);
     }
     // pairs (v[k], v[k+1]) of columns q0 + k, k = 0..8
     auto px = [&](int k) { return (k & 1) ? make_float2(ax[k >> 1].y, ax[(k >> 1) + 1].x) : ax[k >> 1]; };
@@ -423,7 +431,7 @@ __global__ void __launch_bounds__(tile::kThreads) tile_kernel(const __grid_const
         for (int p = 0; p < 4; ++p)
           if (x + p < w) c.nms[(size_t)y * w + x + p] = m[p];
     }
-    *reinterpret_cast<float4*>(nms + r * TW + q) = make_float4(m[0], m[1], m[2], m[3]);
+    *reinterpret_cast<float4*>(nms + r * NS + q) = make_float4(m[0], m[1], m[2], m[3]);
   }
   __syncthreads();
 
@@ -441,10 +449,14 @@ __global__ void __launch_bounds__(tile::kThreads) tile_kernel(const __grid_const
     const int cellx = X / 8 + ccx, celly = Y / 8 + ccy;
     float m = 0.f;
     unsigned idx = 0;
+    // lanes 4g .. 4g+3 and their second elements: four columns of rows g / 2 and g / 2 + 4
+    const float* cell = nms + (ccy * 8 + (g >> 1)) * NS + ccx * 8 + 4 * (g & 1);
+    const float4 e0 = *reinterpret_cast<const float4*>(cell), e1 = *reinterpret_cast<const float4*>(cell + 4 * NS);
+    const float vals[8] = {e0.x, e1.x, e0.y, e1.y, e0.z, e1.z, e0.w, e1.w};
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int f = 4 * g + (k >> 1) + 32 * (k & 1), dy = f >> 3, dx = f & 7;
-      const float v = nms[(ccy * 8 + dy) * TW + ccx * 8 + dx];
+      const float v = vals[k];
       if (v > m) {
         m = v;
         idx = (unsigned)dx | ((unsigned)dy << 16);
@@ -480,8 +492,9 @@ __global__ void __launch_bounds__(tile::kThreads) tile_kernel(const __grid_const
 
   // F. 16x16 sub-tile sums of the response (accumulateGFTT_kernel's reduction order): warp w sums
   //    rows 2w, 2w+1 of each of the 8 sub-tiles, then a 3-level butterfly over the 8 warp sums
-  //    (the eight warp sums share butterflies, three, three and two at a time, each bit-identical to
-  //    its own warp_sum)
+  //    (the eight warp sums by recursive halving: at the first three stages a lane keeps half of its
+  //    partial sums, so value k ends in the lanes whose low bits are k; each addition joins the two
+  //    partial sums that warp_sum joins)
   {
     float v[8];
 #pragma unroll
@@ -491,12 +504,18 @@ __global__ void __launch_bounds__(tile::kThreads) tile_kernel(const __grid_const
       const int x = X + sj * 16 + tx, y = Y + si * 16 + ty;
       v[s8] = (x < w && y < h) ? resp[(si * 16 + ty + 1) * RS + sj * 16 + tx + 1] : 0.f;
     }
-    warp_sum3(v[0], v[1], v[2], lane);
-    warp_sum3(v[3], v[4], v[5], lane);
-    warp_sum2(v[6], v[7], lane);
-    if (lane == 0)
 #pragma unroll
-      for (int s8 = 0; s8 < 8; ++s8) part[s8][wid] = v[s8];
+    for (int st = 0; st < 3; ++st) {
+      const bool up = (lane >> st) & 1;
+#pragma unroll
+      for (int k = 0; k < (4 >> st); ++k) {
+        const float keep = up ? v[2 * k + 1] : v[2 * k], send = up ? v[2 * k] : v[2 * k + 1];
+        v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 1 << st);
+      }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 8);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+    if (lane < 8) part[lane][wid] = v[0];
   }
   __syncthreads();
   {
