@@ -611,7 +611,8 @@ __device__ void box3_tile(const uint8_t* raw, uint8_t* out, int a0x, int a0y, in
   }
 }
 
-// Image and gradients of the tile's level-1 and level-2 cores from their shared-memory regions.
+// Image and gradients of the tile's level-1 and level-2 cores from their shared-memory regions (no grad_y
+// where a level has no such plane: a current or secondary pyramid may come without them).
 template <int T2>
 __device__ __forceinline__ void levels12_outputs(const Level& L1, const Level& L2, const float* B1, const float* B2,
                                                  int X2, int Y2, int tid) {
@@ -662,12 +663,12 @@ __device__ __forceinline__ void levels12_outputs(const Level& L1, const Level& L
     if (x + 3 < L.w) {
       *reinterpret_cast<float4*>(L.img + o) = make_float4(v[4], v[5], v[6], v[7]);
       *reinterpret_cast<float4*>(L.gx + o) = make_float4(gx[0], gx[1], gx[2], gx[3]);
-      *reinterpret_cast<float4*>(L.gy + o) = make_float4(gy[0], gy[1], gy[2], gy[3]);
+      if (L.gy) *reinterpret_cast<float4*>(L.gy + o) = make_float4(gy[0], gy[1], gy[2], gy[3]);
     } else {
       for (int i = 0; i < 4 && x + i < L.w; ++i) {
         L.img[o + i] = v[4 + i];
         L.gx[o + i] = gx[i];
-        L.gy[o + i] = gy[i];
+        if (L.gy) L.gy[o + i] = gy[i];
       }
     }
   }
