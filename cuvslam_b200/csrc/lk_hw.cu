@@ -291,7 +291,8 @@ __global__ void __launch_bounds__(32) lk_hw_kernel(const __grid_constant__ LkLau
     return;
   }
   track_hw<HORIZ, COUNT, true>(cam, T, td, thr, cam.retrack_ncc, none, fork, lane, p.counts);
-  if (fork.level < 0) return;
+  // (a track whose radius is not a number has no second pass)
+  if (fork.level < 0 || !(td.search_radius_px >= 0.f)) return;
   __syncwarp();
   if (td.track_status != 0) return;
   if (fork.level == 0) {
