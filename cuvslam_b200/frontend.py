@@ -166,8 +166,8 @@ def tracks_to_device(tracks, device="cuda"):
     cuda_kernels.h:76-87)."""
     arr = np.ascontiguousarray(tracks, dtype=TRACK_DTYPE)
     raw = arr.view(np.uint8).reshape(len(arr), 80)
-    if not raw.flags.writeable or torch.device(device).type == "cpu":
-        raw = raw.copy()  # (the copy to a device is the tensor's own memory)
+    if not raw.flags.writeable or device is None or torch.device(device).type == "cpu":
+        raw = raw.copy()  # (the copy to a device is the tensor's own memory; None stays on the host)
     return torch.from_numpy(raw).to(device)
 
 
