@@ -25,11 +25,17 @@ from .types import TRACK_DTYPE
 DEFAULT_LK_SAMPLING = _lib.FE_SAMPLE_HARDWARE
 
 
+# A Stream object made only to read its handle costs more than many a call; torch's raw getter is not part of
+# its public interface, so a torch without it takes the object.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_handle(stream=None):
-    """The stream's handle, or the current device's current stream's (without a Stream object made for it)."""
-    if stream is not None:
-        return ctypes.c_void_p(stream.cuda_stream)
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    """The stream's handle, or the current device's current stream's (after torch's own check that CUDA can be
+    used in this process)."""
+    if stream is None and _raw_stream is not None:
+        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
+    return ctypes.c_void_p((stream if stream is not None else torch.cuda.current_stream()).cuda_stream)
 
 
 def _ptr(t):
