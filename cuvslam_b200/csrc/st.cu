@@ -347,14 +347,14 @@ struct State {
 };
 
 // Gauss-Newton refinement against the previous patch; false when a patch leaves the level or a
-// solve fails (or_st refine()).
-template <int SAMPLING>
+// solve fails (or_st refine()).  SHIFT: some steps are shift steps.
+template <int SAMPLING, bool SHIFT>
 __device__ bool refine(const Level& L, const float* prev, float prev_sum, int n_shift, int n_full, const Taps& T,
                        int lane, State& s) {
   float m[4] = {s.m[0], s.m[1], s.m[2], s.m[3]};
   float cx = s.cx, cy = s.cy;
   for (int it = 0; it < n_shift + n_full; ++it) {
-    const bool full = it >= n_shift;
+    const bool full = !SHIFT || it >= n_shift;
     if (!inside(cx, cy, L.w, L.h)) return false;
     float sx[3], sy[3], p[3], gx[3], gy[3], r[3];
     if (!current_coords(L, cx, cy, m, T, sx, sy)) return false;
@@ -380,10 +380,9 @@ __device__ bool refine(const Level& L, const float* prev, float prev_sum, int n_
       gy[e] = __fsub_rn(gy[e], gym);
       r[e] = __fsub_rn(__fsub_rn(p[e], prev[e]), delta);
     }
-    float part[24];
-#pragma unroll
-    for (int k = 0; k < 24; ++k) part[k] = 0.f;
+    float sxx, sxy, syy, rx, ry, slot = 0.f;
     if (full) {
+      float part[24];
 #pragma unroll
       for (int k = 1; k < 6; ++k) {
 #pragma unroll
@@ -405,15 +404,28 @@ __device__ bool refine(const Level& L, const float* prev, float prev_sum, int n_
         part[15 + k] = LANE_SUM(
             T, __fmul_rn(__fmul_rn(r[e], __fmul_rn(k < 2 ? (float)(T.ix[e] - 4) : (float)(T.iy[e] - 4), T.wt[e])),
                          (k % 2 == 0) ? gx[e] : gy[e]));
+      part[19] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gx[e]), gx[e]));
+      part[20] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gx[e]), gy[e]));
+      part[21] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gy[e]), gy[e]));
+      part[22] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], r[e]), gx[e]));
+      part[23] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], r[e]), gy[e]));
+      slot = reduce_scatter(part, lane);
+      sxx = __shfl_sync(kFull, slot, 19);
+      sxy = __shfl_sync(kFull, slot, 20);
+      syy = __shfl_sync(kFull, slot, 21);
+      rx = __shfl_sync(kFull, slot, 22);
+      ry = __shfl_sync(kFull, slot, 23);
+    } else {
+      // (a shift step has five sums; as five of the full step's 24 they made 20 shift steps of 8191 tracks take
+      // 210 us for 200)
+      sxx = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gx[e]), gx[e]));
+      sxy = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gx[e]), gy[e]));
+      syy = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gy[e]), gy[e]));
+      rx = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], r[e]), gx[e]));
+      ry = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], r[e]), gy[e]));
+      warp_sum3(sxx, sxy, syy, lane);
+      warp_sum2(rx, ry, lane);
     }
-    part[19] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gx[e]), gx[e]));
-    part[20] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gx[e]), gy[e]));
-    part[21] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], gy[e]), gy[e]));
-    part[22] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], r[e]), gx[e]));
-    part[23] = LANE_SUM(T, __fmul_rn(__fmul_rn(T.wt[e], r[e]), gy[e]));
-    const float slot = reduce_scatter(part, lane);
-    const float sxx = __shfl_sync(kFull, slot, 19), sxy = __shfl_sync(kFull, slot, 20),
-                syy = __shfl_sync(kFull, slot, 21), rx = __shfl_sync(kFull, slot, 22), ry = __shfl_sync(kFull, slot, 23);
     const float det = __fsub_rn(__fmul_rn(sxx, syy), __fmul_rn(sxy, sxy));
     const float nx = __fsub_rn(__fmul_rn(syy, rx), __fmul_rn(sxy, ry));
     const float ny = __fsub_rn(__fmul_rn(sxx, ry), __fmul_rn(sxy, rx));
@@ -469,7 +481,7 @@ __device__ __forceinline__ void up(float& x, float& y) {
 }
 
 // One track (st_track_kernel / st_track_with_cache_kernel).
-template <int SAMPLING, bool CACHED>
+template <int SAMPLING, bool CACHED, bool SHIFT>
 __device__ void track_one(const StLaunch& P, fe_track_data& td, const Taps& T, int lane) {
   const fe_affine_cache* cd = nullptr;
   if (CACHED) {
@@ -531,7 +543,7 @@ __device__ void track_one(const StLaunch& P, fe_track_data& td, const Taps& T, i
     }
     __syncwarp();
     if (lane < 4) td.info[lane] = (lane == 0 || lane == 3) ? 1.f / 9.f : 0.f;
-    const bool ok = have && refine<SAMPLING>(L, prev, prev_sum, P.n_shift, P.n_full, T, lane, s);
+    const bool ok = have && refine<SAMPLING, SHIFT>(L, prev, prev_sum, P.n_shift, P.n_full, T, lane, s);
     if (!ok) {
       if (level > 0) {
         up(s.cx, s.cy);
@@ -587,8 +599,10 @@ __device__ void track_one(const StLaunch& P, fe_track_data& td, const Taps& T, i
 }
 
 // Persistent warps: each takes the next track from P.counter (zeroed before the launch).
-// MINB: blocks per SM the registers are budgeted for.
-template <int SAMPLING, bool CACHED, int MINB>
+// MINB: blocks per SM the registers are budgeted for.  SHIFT: the call has shift steps (without them the step
+// needs neither their branch nor its registers: 8191 tracks of a 1280x720 pair with 20 full steps take 1125 us,
+// 1180 in the kernel that has both; 30000 take 3413 and 3579).
+template <int SAMPLING, bool CACHED, bool SHIFT, int MINB>
 __global__ void __launch_bounds__(kWarps * 32, MINB) st_track_kernel(const __grid_constant__ StLaunch P) {
   const int lane = threadIdx.x & 31;
   const Taps T = make_taps(lane);
@@ -597,7 +611,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) st_track_kernel(const __gri
     if (lane == 0) g = atomicAdd(P.counter, 1);
     g = __shfl_sync(kFull, g, 0);
     if (g >= P.n) return;
-    track_one<SAMPLING, CACHED>(P, P.tracks[g], T, lane);
+    track_one<SAMPLING, CACHED, SHIFT>(P, P.tracks[g], T, lane);
     __syncwarp();
   }
 }
@@ -643,19 +657,20 @@ __global__ void __launch_bounds__(kWarps * 32) st_build_kernel(const __grid_cons
 }
 
 // Blocks resident on the device (persistent grid), found once per process.
-template <int SAMPLING, bool CACHED, int MINB>
+template <int SAMPLING, bool CACHED, bool SHIFT, int MINB>
 int resident_blocks() {
   static const int resident = [] {
     int per_sm = 0, dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, st_track_kernel<SAMPLING, CACHED, MINB>, kWarps * 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, st_track_kernel<SAMPLING, CACHED, SHIFT, MINB>, kWarps * 32,
+                                                  0);
     return (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
   }();
   return resident;
 }
 
-template <int SAMPLING, bool CACHED>
+template <int SAMPLING, bool CACHED, bool SHIFT>
 cudaError_t launch_track(const StLaunch& p, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(p.counter, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
@@ -663,19 +678,21 @@ cudaError_t launch_track(const StLaunch& p, cudaStream_t s) {
   // the chain of steps sets the time: 438 us there, 486 at three blocks (80 registers) with 150 tracks,
   // 586 and 714 with 2400, 1029 both with 4800.  Past that the third block's warps pay: 1519 us against
   // 1568 with 8191.
-  const int blocks = (p.n + kWarps - 1) / kWarps, two = resident_blocks<SAMPLING, CACHED, 2>();
+  const int blocks = (p.n + kWarps - 1) / kWarps, two = resident_blocks<SAMPLING, CACHED, SHIFT, 2>();
   if (2 * blocks <= 3 * two)
-    st_track_kernel<SAMPLING, CACHED, 2><<<min(blocks, two), kWarps * 32, 0, s>>>(p);
+    st_track_kernel<SAMPLING, CACHED, SHIFT, 2><<<min(blocks, two), kWarps * 32, 0, s>>>(p);
   else
-    st_track_kernel<SAMPLING, CACHED, 3>
-        <<<min(blocks, resident_blocks<SAMPLING, CACHED, 3>()), kWarps * 32, 0, s>>>(p);
+    st_track_kernel<SAMPLING, CACHED, SHIFT, 3>
+        <<<min(blocks, resident_blocks<SAMPLING, CACHED, SHIFT, 3>()), kWarps * 32, 0, s>>>(p);
   return cudaGetLastError();
 }
 
 template <int SAMPLING>
 cudaError_t launch_sampling(const StLaunch& p, int kind, cudaStream_t s) {
-  if (kind == 0) return launch_track<SAMPLING, false>(p, s);
-  if (kind == 1) return launch_track<SAMPLING, true>(p, s);
+  if (kind == 0)
+    return p.n_shift > 0 ? launch_track<SAMPLING, false, true>(p, s) : launch_track<SAMPLING, false, false>(p, s);
+  if (kind == 1)
+    return p.n_shift > 0 ? launch_track<SAMPLING, true, true>(p, s) : launch_track<SAMPLING, true, false>(p, s);
   st_build_kernel<SAMPLING><<<(p.n + kWarps - 1) / kWarps, kWarps * 32, 0, s>>>(p);
   return cudaGetLastError();
 }
