@@ -171,8 +171,10 @@ __device__ void stage_tail(const Level& src, const Level* tail, int n, float* sm
   }
 }
 
+// (five blocks per SM: the straight-line edge path takes 54 registers unbounded, with which four blocks fit and a
+// two-level build of a 4096x4096 uint8 frame takes 461 us; 407 us at 48 registers, 418 with the edges in a loop)
 template <typename InT, int NL, int KT>
-__global__ void __launch_bounds__(kThreads) pyramid_stage_kernel(const __grid_constant__ StageBatch batch) {
+__global__ void __launch_bounds__(kThreads, 5) pyramid_stage_kernel(const __grid_constant__ StageBatch batch) {
   extern __shared__ float smem[];
   // camera of this CTA: last job whose tile_begin <= blockIdx.x
   int lo = 0, hi = batch.njobs - 1;
