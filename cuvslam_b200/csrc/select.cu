@@ -797,20 +797,112 @@ __global__ void __launch_bounds__(256) bin_kernel(const __grid_constant__ Batch 
 }
 
 // ---------------------------------------------------------------- final order
-// A camera's kept keys are distinct, so a key's place in their order is the number of smaller ones: a
-// block ranks 32 keys, eight threads each over an eighth of all keys, and writes them out.  The count is
-// quadratic but spread over the device: 4 us for 1600 keys of one camera and 19 us for 32 cameras (11 and 42 us as one block's
-// bitonic sort per camera).
-constexpr int kRankKeys = 32, kRankChunk = 2048;
+// A camera's kept keys are distinct, so a key's place in their order is the number of smaller ones: a block
+// ranks 32 keys, eight threads each over an eighth of all keys, and writes them out.  The count is quadratic
+// but spread over the device: 4 us for 1600 keys of one camera and 19 us for 32 cameras of 300-3000 (11 and
+// 42 us as one block's bitonic sort per camera).
+//
+// Where the launch's cameras may have more than kRankWork comparisons to make, sort_chunks_kernel first sorts
+// every kRankChunk keys of a camera that has more by a block of its own, and a key's rank is the sum of its
+// places in the chunks, found by binary search; the keys of a warp are neighbours, so their searches read the
+// same lines.  Selection part of 1920x1200 cameras, by counting alone and by chunks: 2 x 6000 features 92 and
+// 95 us, 2 x 8000 107 and 96, 8 x 3000 196 and 199, 8 x 8000 297 and 203, 32 x 2500 641 and 620, 32 x 16000
+// 2495 and 658 (829 with one block's sort per camera).
+constexpr int kRankKeys = 32, kRankChunk = 2048, kRankThreads = kRankKeys * 8;
+constexpr int kMaxChunks = kMaxSelectKeys / kRankChunk;
+constexpr int64_t kRankWork = 1 << 27;
+
+__device__ __forceinline__ int kept_keys(const SelectCam& c, int key_cap) {
+  return min(min(c.stats[2], c.q_cap), key_cap);
+}
+
+// Ascending bitonic sort of n_pow2 (a power of two) keys in shared memory by the whole block
+// (blockDim.x a multiple of 32).  Compare-exchange steps whose partner index i ^ j lies in the same
+// run of 32 keys (j <= 16) run in registers, lane i of a warp holding key i of its run and swapping
+// through shuffles, so the block meets at a barrier once per merge width k for them instead of once
+// per step; wider steps exchange through shared memory.  The network is the same, so is the result.
+template <typename K>
+__device__ void block_bitonic_sort(K* keys, int n_pow2) {
+  const int lane = threadIdx.x & 31;
+  for (int k = 2; k <= n_pow2; k <<= 1) {
+    for (int j = k >> 1; j >= 32; j >>= 1) {
+      for (int i = threadIdx.x; i < n_pow2; i += blockDim.x) {
+        const int ixj = i ^ j;
+        if (ixj > i) {
+          const K a = keys[i], bb = keys[ixj];
+          const bool up = (i & k) == 0;
+          if ((a > bb) == up) {
+            keys[i] = bb;
+            keys[ixj] = a;
+          }
+        }
+      }
+      __syncthreads();
+    }
+    // steps j = min(k/2, 16) .. 1: the lower index of a pair keeps the smaller key when the run of
+    // width k ascends ((i & k) == 0) and the larger one when it descends
+    for (int base = (int)(threadIdx.x & ~31u); base < n_pow2; base += blockDim.x) {
+      const int i = base + lane;
+      K v = i < n_pow2 ? keys[i] : K(0);
+      const bool up = (i & k) == 0;
+      for (int j = min(k >> 1, 16); j > 0; j >>= 1) {
+        const K o = __shfl_xor_sync(0xffffffffu, v, j);
+        const bool lower = (lane & j) == 0;
+        v = (lower == up) ? (o < v ? o : v) : (o > v ? o : v);
+      }
+      if (i < n_pow2) keys[i] = v;
+    }
+    __syncthreads();
+  }
+}
 
 template <typename Batch>
-__global__ void __launch_bounds__(kRankKeys * 8) final_kernel(const __grid_constant__ Batch b, int key_cap) {
+__global__ void __launch_bounds__(1024) sort_chunks_kernel(const __grid_constant__ Batch b, int key_cap) {
   __shared__ uint64_t keys[kRankChunk];
   const SelectCam& c = b.cam[blockIdx.y];
-  const int n = min(min(c.stats[2], c.q_cap), key_cap), out = min(n, wanted_features(c));
+  const int n = kept_keys(c, key_cap), base = blockIdx.x * kRankChunk, m = min(kRankChunk, n - base);
+  if (n <= kRankChunk || m <= 0) return;  // block-uniform
+  int np = 1;
+  while (np < m) np <<= 1;
+  for (int i = threadIdx.x; i < np; i += blockDim.x) keys[i] = i < m ? c.q_keys[base + i] : ~0ull;
+  __syncthreads();
+  block_bitonic_sort(keys, np);
+  for (int i = threadIdx.x; i < m; i += blockDim.x) c.q_keys[base + i] = keys[i];
+}
+
+// sorted: sort_chunks_kernel ran before.
+template <typename Batch>
+__global__ void __launch_bounds__(kRankThreads) final_kernel(const __grid_constant__ Batch b, int key_cap, bool sorted) {
+  __shared__ uint64_t keys[kRankChunk];
+  const SelectCam& c = b.cam[blockIdx.y];
+  const int n = kept_keys(c, key_cap), out = min(n, wanted_features(c));
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     if (c.stats[2] > key_cap) atomicOr(&c.stats[3], 4);
     *c.out_count = out;
+  }
+  auto put = [&](uint64_t key, int rank) {
+    if (rank >= out) return;
+    const float2 p = c.cell_xy[(int)(key & 0xffffffffu)];
+    c.out_xy[2 * rank] = p.x;
+    c.out_xy[2 * rank + 1] = p.y;
+  };
+  if (sorted && n > kRankChunk) {
+    const int i = blockIdx.x * kRankThreads + threadIdx.x;
+    if (i >= n) return;
+    const uint64_t mine = c.q_keys[i];
+    int less[kMaxChunks] = {};  // keys of each chunk that are smaller
+#pragma unroll
+    for (int step = kRankChunk; step > 0; step >>= 1)
+#pragma unroll
+      for (int q = 0; q < kMaxChunks; ++q) {
+        const int at = q * kRankChunk + less[q] + step;  // the key before it decides
+        if (at <= min(n, (q + 1) * kRankChunk) && c.q_keys[at - 1] < mine) less[q] += step;
+      }
+    int rank = 0;
+#pragma unroll
+    for (int q = 0; q < kMaxChunks; ++q) rank += less[q];
+    put(mine, rank);
+    return;
   }
   if ((int)blockIdx.x * kRankKeys >= n) return;  // block-uniform
   const int part = threadIdx.x & 7, i = blockIdx.x * kRankKeys + (threadIdx.x >> 3);
@@ -826,11 +918,7 @@ __global__ void __launch_bounds__(kRankKeys * 8) final_kernel(const __grid_const
   }
 #pragma unroll
   for (int d = 1; d < 8; d <<= 1) rank += __shfl_xor_sync(0xffffffffu, rank, d);
-  if (part == 0 && i < n && rank < out) {
-    const float2 p = c.cell_xy[(int)(mine & 0xffffffffu)];
-    c.out_xy[2 * rank] = p.x;
-    c.out_xy[2 * rank + 1] = p.y;
-  }
+  if (part == 0 && i < n) put(mine, rank);
 }
 
 }  // namespace
@@ -870,10 +958,21 @@ namespace {
 template <typename Batch>
 cudaError_t launch_bins_final(const Batch& b, int bin_key_cap, int final_key_cap, cudaStream_t s) {
   bin_kernel<<<dim3(64, b.ncams), 256, sizeof(uint64_t) * bin_key_cap, s>>>(b, bin_key_cap);
-  int q_cap = 1;
-  for (int i = 0; i < b.ncams; ++i) q_cap = max(q_cap, b.cam[i].q_cap);
-  final_kernel<<<dim3((min(q_cap, final_key_cap) + kRankKeys - 1) / kRankKeys, b.ncams), kRankKeys * 8, 0, s>>>(
-      b, final_key_cap);
+  int q_cap = 1, most = 0;
+  int64_t work = 0;
+  for (int i = 0; i < b.ncams; ++i) {
+    const SelectCam& c = b.cam[i];
+    // the bins' quotas add up to the features that a camera should have in all, and their roundings
+    const int n = c.target_total > 0 ? min(c.q_cap, c.target_total + 64) : c.q_cap;
+    q_cap = max(q_cap, c.q_cap);
+    most = max(most, n);
+    work += (int64_t)n * n;
+  }
+  q_cap = min(q_cap, final_key_cap);
+  const bool sorted = most > kRankChunk && work > kRankWork;
+  if (sorted)
+    sort_chunks_kernel<<<dim3((q_cap + kRankChunk - 1) / kRankChunk, b.ncams), 1024, 0, s>>>(b, final_key_cap);
+  final_kernel<<<dim3((q_cap + kRankKeys - 1) / kRankKeys, b.ncams), kRankThreads, 0, s>>>(b, final_key_cap, sorted);
   return cudaGetLastError();
 }
 
