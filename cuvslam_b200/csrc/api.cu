@@ -578,8 +578,8 @@ int fe_pyramid_init(void* device_memory, int64_t bytes, int width, int height, i
   return FE_OK;
 }
 
-// The pyramid of a level 0 already in pyr->image[0] (the input stage wrote it): the FP32 plan, whose
-// first stage rewrites level 0 with the same values while it computes the gradients.
+// The pyramid of a level 0 already in pyr->image[0] (the input stage wrote it): the FP32 plan.  With three levels
+// or more its first stage leaves level 0's image as it is (keep_level0), with fewer it rewrites the same values.
 int build_from_level0(fe_context* ctx, const fe_pyramid* pyr, cudaStream_t s) {
   StagePlan plan;
   int rc = plan_pyramid(pyr->image[0], pyr->pitch_bytes[0], false, *pyr, plan);

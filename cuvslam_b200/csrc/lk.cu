@@ -94,7 +94,8 @@ cudaError_t launch_shape(const LkLaunch& p, cudaStream_t s) {
     int per_sm = 0, dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lk_kernel<SAMPLING, HORIZ, MODE, WARPS, MINB>, WARPS * 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lk_kernel<SAMPLING, HORIZ, MODE, WARPS, MINB>, WARPS * 32,
+                                                  0);
     return (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
   }();
   int blocks = (p.total + WARPS - 1) / WARPS;
@@ -104,10 +105,10 @@ cudaError_t launch_shape(const LkLaunch& p, cudaStream_t s) {
 }
 
 // Reference-rule launches take the block shape p.shape (kLkShapes); the differentiable modes use
-// the first.
+// the first (and compile no other).
 template <int SAMPLING, bool HORIZ, int MODE>
 cudaError_t launch(const LkLaunch& p, cudaStream_t s) {
-  if (MODE == kModeRef || MODE == kModeRetrack) {
+  if constexpr (MODE == kModeRef || MODE == kModeRetrack) {
     switch (p.shape) {
       case 1: return launch_shape<SAMPLING, HORIZ, MODE, 8, 3>(p, s);
       case 2: return launch_shape<SAMPLING, HORIZ, MODE, 4, 8>(p, s);

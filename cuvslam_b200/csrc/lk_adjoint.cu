@@ -711,7 +711,8 @@ __global__ void bin_kernel(const __grid_constant__ AdjGather G) {
 }
 
 // Exclusive prefix sum of the per-tile counts (one CTA, sixteen tiles per thread per pass: a pass is a
-// chain of loads, shuffles and barriers, so fewer and wider ones are faster); clears the fill cursors and lists the tiles with more than kWarpList records.
+// chain of loads, shuffles and barriers, so fewer and wider ones are faster); clears the fill cursors and
+// lists the tiles with more than kWarpList records.
 __global__ void __launch_bounds__(1024) scan_kernel(const __grid_constant__ AdjGather G) {
   __shared__ int warp_tot[32];
   __shared__ int carry;

@@ -88,8 +88,8 @@ __device__ __forceinline__ float downscale_px(const float* src, int stride, int 
 // (row length `stride`) whose origin is (ax, ay): each takes the value the mirror addressing reads
 // there (-x-1 / 2n-x-1), so that the decimation's taps need no index arithmetic near the edges.  A
 // frame's time is that of its slowest tile where all tiles run at once: the mirrored path per pixel
-// made a corner tile four times as long as an inner one (levels 1-2 of the FP32 stage 21 500 cycles, now
-// 4 700; one 640x480 uint8 frame 26.6 us, now 16.5).
+// made a corner tile four times as long as an inner one (levels 1-2 of the FP32 stage 21 500 cycles,
+// 4 700 with the cells in place).
 template <int NT, typename T>
 __device__ __forceinline__ void mirror_rings(T* buf, int stride, int rw, int rh, int ax, int ay, int w, int h,
                                              int tid) {
@@ -1411,7 +1411,7 @@ __global__ void input_mono_kernel(const uint8_t* src, int64_t pitch, int box3, i
 // RGB frame: a thread takes four pixels of four rows; each row's 18 bytes (pixels x - 1 .. x + 4) come as
 // six aligned words shifted into place, single bytes near the frame's ends; the prefilter's horizontal
 // sums slide down the rows.  (A thread per pixel that read its nine neighbours' 27 bytes one by one took
-// 18.9 us for 1921x1201 with the prefilter, this about 7 us.)
+// 18.9 us for 1921x1201 with the prefilter, this 8.4 us.)
 constexpr int kRgbRows = 4;
 
 __global__ void __launch_bounds__(256) input_rgb_kernel(const uint8_t* src, int64_t pitch, int box3, int w, int h,

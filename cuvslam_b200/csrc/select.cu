@@ -93,8 +93,8 @@ __device__ __forceinline__ void count_bin(const SelectCam& c, float x, float y, 
 
 // A thread per (feature, window row): the order of the features matters only to the rule that no more
 // than `cells` of them burn, so this serves every camera with no more features than cells.  Spread over
-// the device it takes 2.2 us for 600 features and 6 us for 32 cameras of 300-3000 (one block per camera that ranked them and burned nine rows
-// a thread took 6 us for 600 features and 20 us for 32 cameras of 300-3000).
+// the device it takes 2.2 us for 600 features and 6.5 us for 32 cameras of 300-3000 (one block per camera
+// that ranked them and burned nine rows a thread took 6 and 20 us).
 template <typename Batch>
 __global__ void __launch_bounds__(288) alive_kernel(const __grid_constant__ Batch b) {
   const SelectCam& c = b.cam[blockIdx.y];
@@ -872,7 +872,8 @@ __global__ void __launch_bounds__(1024) sort_chunks_kernel(const __grid_constant
 
 // sorted: sort_chunks_kernel ran before.
 template <typename Batch>
-__global__ void __launch_bounds__(kRankThreads) final_kernel(const __grid_constant__ Batch b, int key_cap, bool sorted) {
+__global__ void __launch_bounds__(kRankThreads)
+    final_kernel(const __grid_constant__ Batch b, int key_cap, bool sorted) {
   __shared__ uint64_t keys[kRankChunk];
   const SelectCam& c = b.cam[blockIdx.y];
   const int n = kept_keys(c, key_cap), out = min(n, wanted_features(c));
@@ -934,7 +935,8 @@ int select_tile_h() { return tile::TH; }
 namespace {
 template <typename Batch>
 cudaError_t set_attrs() {
-  cudaError_t e = cudaFuncSetAttribute(tile_kernel<false, Batch>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile::kSmem);
+  cudaError_t e = cudaFuncSetAttribute(tile_kernel<false, Batch>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       tile::kSmem);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(bin_kernel<Batch>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(sizeof(uint64_t) * kMaxSelectKeys));
