@@ -20,12 +20,13 @@
 // so each reflector and norm update runs once per column in parallel.  Operations are unfused
 // (__fmul_rn / __fadd_rn) so the oracle restates them exactly.
 //
-// Bound by issue with many tracks and by a track's chain of steps with few (a step of one warp alone:
-// 10 800 cycles before the sums shared a butterfly, the QR's steps were unrolled and its pivot found by a
-// warp maximum, 6 400 of them in the QR).  1920x1200, 20 full steps a level: 150 tracks 574 -> 438 us,
-// 2400 tracks 852 -> 586, 8191 tracks 1716 -> 1519.  Several tracks per warp or block with their QR solves
-// side by side were slower (1.8-5.1 ms at 8191): their code and their barriers cost more than the idle
-// lanes of one solve.
+// A track's chain of steps sets the time with few tracks (a step of one warp alone: 10 800 cycles before the
+// sums shared a butterfly, the QR's steps were unrolled and its pivot found by a warp maximum, 6 400 of them in
+// the QR); with many the warps share the issue slots, of which 61 % are used at 20 warps per SM (a warp's
+// issued instruction waits 2.0 cycles for the one before, 1.2 on loads, 1.0 for instructions).  1920x1200, 20
+// full steps a level: 150 tracks 600 -> 454 us, 2400 854 -> 586, 8191 1720 -> 1470.  Several tracks per warp
+// or block with their QR solves side by side were slower (1.8-5.1 ms at 8191): their code and their barriers
+// cost more than the idle lanes of one solve.
 #include <cuda_runtime.h>
 
 #include "fe_common.cuh"
@@ -674,12 +675,12 @@ template <int SAMPLING, bool CACHED, bool SHIFT>
 cudaError_t launch_track(const StLaunch& p, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(p.counter, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
-  // While a warp at two blocks per SM (128 registers, no spills) has hardly more than a track of its own
-  // the chain of steps sets the time: 438 us there, 486 at three blocks (80 registers) with 150 tracks,
-  // 586 and 714 with 2400, 1029 both with 4800.  Past that the third block's warps pay: 1519 us against
-  // 1568 with 8191.
+  // While a warp at two blocks per SM (128 registers, no spills) has hardly more than a track of its own the
+  // chain of steps sets the time; past that the third block's warps pay (80 registers).  1920x1200, 20 full
+  // steps, two and three blocks: 150 tracks 455 and 490 us, 2400 582 and 670, 2960 733 and 740, 3552 830 and
+  // 751, 8191 1530 and 1454.
   const int blocks = (p.n + kWarps - 1) / kWarps, two = resident_blocks<SAMPLING, CACHED, SHIFT, 2>();
-  if (2 * blocks <= 3 * two)
+  if (4 * blocks <= 5 * two)
     st_track_kernel<SAMPLING, CACHED, SHIFT, 2><<<min(blocks, two), kWarps * 32, 0, s>>>(p);
   else
     st_track_kernel<SAMPLING, CACHED, SHIFT, 3>
