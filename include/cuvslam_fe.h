@@ -173,7 +173,8 @@ FE_API int fe_build_pyramid(fe_context* ctx, const uint8_t* image, int64_t image
 FE_API int fe_build_pyramid_rgb(fe_context* ctx, const uint8_t* image, int64_t image_pitch_bytes, int width,
                                 int height, int box3, const fe_pyramid* pyr, fe_stream stream);
 /* Same from an FP32 level-0 image (rows pitch_bytes apart): GaussianGPUImagePyramid::build of a
- * float GPUImageT (image_pyramid.h:81-98) + GPUGradientPyramid::set (gradient_pyramid.cpp:83-118). */
+ * float GPUImageT (image_pyramid.h:81-98) + GPUGradientPyramid::set (gradient_pyramid.cpp:83-118).
+ * A level's grad_y may be NULL here (a pyramid that is only tracked into): that plane is left out. */
 FE_API int fe_build_pyramid_f32(fe_context* ctx, const float* image, int64_t image_pitch_bytes, int width, int height,
                          const fe_pyramid* pyr, fe_stream stream);
 
